@@ -23,6 +23,25 @@ __device__ __forceinline__ void set3(float3& v, int a, float x) {
   if (a == 0) v.x = x; else if (a == 1) v.y = x; else v.z = x;
 }
 
+// acc + a * c per component, one rounding each
+__device__ __forceinline__ float3 fma3(const float3 a, float c, const float3 acc) {
+  return make_float3(__fmaf_rn(a.x, c, acc.x), __fmaf_rn(a.y, c, acc.y), __fmaf_rn(a.z, c, acc.z));
+}
+__device__ __forceinline__ float dot3_rn(const float3 a, const float3 b) {
+  return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)));
+}
+__device__ __forceinline__ float3 scaled(const float3 a, float c) {
+  return make_float3(__fmul_rn(a.x, c), __fmul_rn(a.y, c), __fmul_rn(a.z, c));
+}
+// |a|^2 of a move, in the order x and y first
+__device__ __forceinline__ float square_rn(const float3 a) {
+  return __fmaf_rn(a.z, a.z, __fmaf_rn(a.x, a.x, __fmul_rn(a.y, a.y)));
+}
+// x* = fl(x + displacement), one rounding per component wherever it is formed.
+__device__ __forceinline__ float3 displaced(const float3 x, const float3 d) {
+  return make_float3(__fadd_rn(x.x, d.x), __fadd_rn(x.y, d.y), __fadd_rn(x.z, d.z));
+}
+
 // Exactly rounded |a - b|^2 with no contraction: the neighbour predicate of
 // particles.cpp:260 evaluated in FP32 (a host check can repeat it bit for bit).
 __device__ __forceinline__ float dist2_rn(const float4& a, const float4& b) {
@@ -86,9 +105,10 @@ __device__ __forceinline__ float wall_value(const SceneDesc& sc, int wall) {
 }
 
 // applyForceVelocity (particles.cpp:180, v += g dt) and the predicted move v dt.
+// Every rounding is explicit, so no caller's arithmetic is contracted with it.
 __device__ __forceinline__ float3 predict_delta(const float4& v4, const DevParams& P, float dt) {
-  const float3 v = make_float3(v4.x + P.g[0] * dt, v4.y + P.g[1] * dt, v4.z + P.g[2] * dt);
-  return v * dt;
+  return make_float3(__fmul_rn(__fmaf_rn(P.g[0], dt, v4.x), dt), __fmul_rn(__fmaf_rn(P.g[1], dt, v4.y), dt),
+                     __fmul_rn(__fmaf_rn(P.g[2], dt, v4.z), dt));
 }
 
 // Moller-Trumbore test of triangle m (MarchingTriangle::intersect,
@@ -254,7 +274,7 @@ __device__ __forceinline__ bool clear_move(const float3 p, const float3 delta, f
                                            const DevParams& P) {
   if (MESH && (P.n_mesh > 0 || P.n_sph > 0)) return false;
   if (!(s2 > kEps * kEps * 1.001f)) return false;
-  const float3 e = p + delta;
+  const float3 e = displaced(p, delta);
   bool ok = fminf(p.x, e.x) > sc.in_lo[0] && fmaxf(p.x, e.x) < sc.in_hi[0] &&
             fminf(p.y, e.y) > sc.in_lo[1] && fmaxf(p.y, e.y) < sc.in_hi[1] &&
             fminf(p.z, e.z) > sc.in_lo[2] && fmaxf(p.z, e.z) < sc.in_hi[2];
@@ -275,14 +295,15 @@ __device__ __forceinline__ bool clear_move(const float3 p, const float3 delta, f
 // REC additionally writes the collision record to *code (same arithmetic).
 // MESH = false compiles the collider-triangle tests out (for launches with no triangles:
 // they hold registers a neighbour pass would otherwise spend on occupancy).
-// Moves that clear_move accepts take its shortcut.
+// Moves that clear_move accepts take its shortcut. Every rounding of the moves against the box is
+// explicit, so the kernels it is compiled into cannot contract them differently.
 template <bool REC = false, bool MESH = true>
 __device__ __forceinline__ void collide(const float3 x, float3& d, const float3 delta, bool slide,
                                         const SceneDesc& sc, const DevParams& P, uint32_t* code = nullptr) {
-  const float3 p = x + d;
-  const float s2 = delta.x * delta.x + delta.y * delta.y + delta.z * delta.z;
+  const float3 p = displaced(x, d);
+  const float s2 = square_rn(delta);
   if (clear_move<MESH>(p, delta, s2, sc, P)) {
-    d = d + delta;
+    d = displaced(d, delta);
     if (REC) *code = kCollFree;
     return;
   }
@@ -291,7 +312,7 @@ __device__ __forceinline__ void collide(const float3 x, float3& d, const float3 
     if (REC) *code = kCollNone;
     return;
   }
-  const float3 dir = delta * (1.0f / l);
+  const float3 dir = scaled(delta, __fdiv_rn(1.0f, l));
   const float total = l;
   bool intersect = false;
   int clip = 0;
@@ -348,7 +369,7 @@ __device__ __forceinline__ void collide(const float3 x, float3& d, const float3 
     }
   }
   if (wall >= 0 || intersect) {
-    float3 nd = d + dir * t;
+    float3 nd = fma3(dir, t, d);
     if (REC) {
       rc = kCollStop;
       if (wall >= 0) {
@@ -366,12 +387,12 @@ __device__ __forceinline__ void collide(const float3 x, float3& d, const float3 
       if (n_dot > -1.0f) {
         float3 tan = delta;
         set3(tan, a, 0.0f);
-        const float tl = sqrtf(dot3(tan, tan));
+        const float tl = sqrtf(square_rn(tan));
         if (tl > 0.0f) {
-          const float3 dir2 = tan * (1.0f / tl);
-          const float l2 = (total - t) * 0.5f;
+          const float3 dir2 = scaled(tan, __fdiv_rn(1.0f, tl));
+          const float l2 = __fmul_rn(__fsub_rn(total, t), 0.5f);
           int wall2;
-          const float3 p1 = x + nd;
+          const float3 p1 = displaced(x, nd);
           const float t2 = wall_hit(p1, dir2, l2, sc, P.open_mask, &wall2);
           if (MESH && (P.n_mesh > 0 || P.n_sph > 0)) {  // the slide stops at a collider triangle or
                                                         // sphere before the wall
@@ -391,7 +412,7 @@ __device__ __forceinline__ void collide(const float3 x, float3& d, const float3 
               return;
             }
           }
-          nd = nd + dir2 * t2;
+          nd = fma3(dir2, t2, nd);
           if (REC) {
             rc = (rc & ~7u) | kCollSlide;
             if (wall2 >= 0) {
@@ -406,9 +427,9 @@ __device__ __forceinline__ void collide(const float3 x, float3& d, const float3 
     }
     d = nd;
   } else {
-    d = d + delta;
+    d = displaced(d, delta);
   }
-  const float3 q = x + d;
+  const float3 q = displaced(x, d);
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     const float qa = cmp3(q, a);
@@ -718,14 +739,6 @@ __device__ __forceinline__ Pair pair_of(const float4& xi, const float4& xj, floa
   const float hr = fmaxf(__fmaf_rn(-p.r2, rinv, h), 0.0f);
   p.s = p.r2 >= kEps * kEps ? __fmul_rn(__fmul_rn(hr, hr), rinv) : 0.0f;
   return p;
-}
-
-// acc + a * c per component, one rounding each
-__device__ __forceinline__ float3 fma3(const float3 a, float c, const float3 acc) {
-  return make_float3(__fmaf_rn(a.x, c, acc.x), __fmaf_rn(a.y, c, acc.y), __fmaf_rn(a.z, c, acc.z));
-}
-__device__ __forceinline__ float dot3_rn(const float3 a, const float3 b) {
-  return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)));
 }
 
 // Spiky gradient factor s with grad W(r) = spiky_c * s * r (particles.cpp:143-149);

@@ -114,6 +114,9 @@ struct Buffers {
   DevStats* stats = nullptr;
   DevStats* stats_part = nullptr;  // per-block partial records of the stats pass
   unsigned int* err = nullptr;     // sticky PBF_ERRBIT_* word
+  unsigned int* grid_bar = nullptr;  // counters, zero between launches: the whole-step kernel's barrier and the
+                                     // blocks that left it, the statistics pass's ticket
+  int small_sms = 0;                 // SMs for the whole-step kernel (0: not used)
   float* io = nullptr;             // (n, 3) staging for host/device packed transfers
   float* io2 = nullptr;
 };
@@ -222,6 +225,13 @@ cudaError_t launch_step(const Buffers& b, const DevParams& p, const Tuning& t, i
 cudaError_t launch_adjoint(const Buffers& b, const DevParams& p, const Tuning& t, int cur, float dt,
                            const Tape& tape, const float* gx_out, const float* gv_out, float* gx_in,
                            float* gv_in, double* g_rho0, cudaStream_t s);
+// ---- the whole step in one cooperative launch (pbf_small.cu): same results ----
+// small_step_setup: the device's SM count when it can take the launch, else 0. small_step_form: the
+// form that serves the scene, 0 for none (the per-phase kernels).
+cudaError_t small_step_setup(int device, int* sms);
+int small_step_form(const Buffers& b, const DevParams& p);
+cudaError_t launch_step_small(const Buffers& b, const DevParams& p, int form, int cur, float dt, int iters,
+                              bool keep_pred, cudaStream_t s);
 cudaError_t launch_resort(const Buffers& b, const DevParams& p, const Tuning& t, int cur,
                           cudaStream_t s);
 cudaError_t launch_upload(const Buffers& b, int cur, const float* xyz, const float* vel,

@@ -97,6 +97,7 @@ typedef struct pbf_stats {
 #define PBF_ERRBIT_NONFINITE 1u
 #define PBF_ERRBIT_NEIGHBOR_CAPACITY 2u
 #define PBF_ERRBIT_ROW_CAPACITY 4u
+#define PBF_ERRBIT_TIMEOUT 8u /* a bounded wait inside a step gave up (PBF_ERR_TIMEOUT) */
 
 typedef struct pbf_handle pbf_handle;
 
