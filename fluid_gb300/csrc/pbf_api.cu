@@ -185,6 +185,9 @@ void Handle::free_all() {
   if (surf_hash) cudaFree(surf_hash);
   surf_hash = nullptr;
   surf_hash_bytes = 0;
+  if (surf_out) cudaFree(surf_out);
+  surf_out = nullptr;
+  surf_out_bytes = 0;
   if (mesh_dev) cudaFree(mesh_dev);
   mesh_dev = nullptr;
   if (sph_dev) cudaFree(sph_dev);
@@ -283,6 +286,16 @@ pbf_status Handle::ensure_scratch(size_t bytes) {
   scratch_bytes = 0;
   pbf_status st = cuda(cudaMalloc(&scratch, bytes), "cudaMalloc(scratch)");
   if (st == PBF_OK) scratch_bytes = bytes;
+  return st;
+}
+
+pbf_status Handle::ensure_surface_out(size_t bytes) {
+  if (bytes <= surf_out_bytes) return PBF_OK;
+  if (surf_out) cudaFree(surf_out);
+  surf_out = nullptr;
+  surf_out_bytes = 0;
+  pbf_status st = cuda(cudaMalloc(&surf_out, bytes), "cudaMalloc(surface)");
+  if (st == PBF_OK) surf_out_bytes = bytes;
   return st;
 }
 
@@ -951,6 +964,25 @@ void pbf_mc_table(uint16_t* edges, uint8_t* ntri, int8_t* tri) {
 
 namespace pbf {
 
+// Byte offsets of the surface's arrays in the handle's scratch (the field lies at 0).
+struct Handle::SurfScratch {
+  size_t first, tile, axis, any, bytes;
+  uint32_t cubes;
+};
+Handle::SurfScratch Handle::surface_scratch(const SurfGrid& g) const {
+  const size_t cubes = static_cast<size_t>(g.nc[0]) * g.nc[1] * g.nc[2];
+  const size_t corners = static_cast<size_t>(g.nc[0] + 1) * (g.nc[1] + 1) * (g.nc[2] + 1);
+  auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+  SurfScratch w;
+  w.cubes = static_cast<uint32_t>(cubes);
+  w.first = up(4 * corners);
+  w.tile = w.first + up(4 * cubes);
+  w.axis = w.tile + up(4 * (static_cast<size_t>(surface_tiles(w.cubes)) + 1));
+  w.any = w.axis + up(4 * (static_cast<size_t>(g.nc[0]) + g.nc[1] + g.nc[2] + 3));
+  w.bytes = w.any + up(b.n_cells);
+  return w;
+}
+
 // The cube grid of Particles::getSurfacePrims over [lo, hi] (NULL: the reference's fixed
 // bounds, particles.cpp:330-349), the per-cube triangle counts of the current state and
 // their total; the counts stay in the handle's scratch for surface_emit.
@@ -985,17 +1017,12 @@ pbf_status Handle::surface_count(double isolevel, double step, const double* lo,
     st = cuda(cudaMemcpy(surf_table_dev, &surf_table(), sizeof(SurfTable), cudaMemcpyHostToDevice), "H2D table");
     if (st != PBF_OK) return st;
   }
-  const size_t nc = static_cast<size_t>(cubes);
-  const size_t corners = static_cast<size_t>(g->nc[0] + 1) * (g->nc[1] + 1) * (g->nc[2] + 1);
-  const size_t tiles = exclusive_scan_tiles(static_cast<uint32_t>(nc));
-  const size_t naxis = static_cast<size_t>(g->nc[0]) + g->nc[1] + g->nc[2] + 3;
-  st = ensure_scratch(4 * (corners + nc + (nc + 1) + tiles + naxis) + 256);
+  const SurfScratch w = surface_scratch(*g);
+  st = ensure_scratch(w.bytes);
   if (st != PBF_OK) return st;
-  float* field = static_cast<float*>(scratch);
-  uint32_t* cnt = reinterpret_cast<uint32_t*>(field + corners);
-  uint32_t* first = cnt + nc;
-  uint32_t* tile = first + nc + 1;
-  float* axis = reinterpret_cast<float*>(tile + tiles);
+  char* base = static_cast<char*>(scratch);
+  float* axis = reinterpret_cast<float*>(base + w.axis);
+  const size_t naxis = static_cast<size_t>(g->nc[0]) + g->nc[1] + g->nc[2] + 3;
   std::vector<float> ax;
   ax.reserve(naxis);
   for (int a = 0; a < 3; ++a)
@@ -1008,11 +1035,14 @@ pbf_status Handle::surface_count(double isolevel, double step, const double* lo,
   st = cuda(cudaMemcpyAsync(axis, ax.data(), sizeof(float) * naxis, cudaMemcpyHostToDevice, stream), "H2D axis");
   if (st != PBF_OK) return st;
   g->axis = axis;
-  st = cuda(launch_surface_count(b, dp, cur, *g, static_cast<float>(isolevel), surf_table_dev, field, cnt, first,
-                                 tile, stream),
+  uint32_t* tile = reinterpret_cast<uint32_t*>(base + w.tile);
+  st = cuda(launch_surface_count(b, dp, cur, *g, static_cast<float>(isolevel), surf_table_dev,
+                                 reinterpret_cast<uint8_t*>(base + w.any), reinterpret_cast<float*>(base),
+                                 reinterpret_cast<uint32_t*>(base + w.first), tile, stream),
             "surface count");
   if (st != PBF_OK) return st;
-  st = cuda(cudaMemcpyAsync(total, first + nc, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream), "D2H");
+  st = cuda(cudaMemcpyAsync(total, tile + surface_tiles(w.cubes), sizeof(uint32_t), cudaMemcpyDeviceToHost, stream),
+            "D2H");
   if (st == PBF_OK) st = cuda(cudaStreamSynchronize(stream), "sync");
   return st;
 }
@@ -1020,10 +1050,8 @@ pbf_status Handle::surface_count(double isolevel, double step, const double* lo,
 // The first min(cap, total) triangles of the last surface_count into DEVICE arrays.
 pbf_status Handle::surface_emit(const SurfGrid& g, double isolevel, float* xyz, float* nrm, uint32_t cap) {
   if (cap == 0 || b.n == 0) return PBF_OK;
-  const size_t nc = static_cast<size_t>(g.nc[0]) * g.nc[1] * g.nc[2];
-  const size_t corners = static_cast<size_t>(g.nc[0] + 1) * (g.nc[1] + 1) * (g.nc[2] + 1);
-  const float* field = static_cast<const float*>(scratch);
-  const uint32_t* first = reinterpret_cast<const uint32_t*>(field + corners) + nc;
+  const SurfScratch w = surface_scratch(g);
+  const char* base = static_cast<const char*>(scratch);
   if (cap > (1u << 28)) return fail(PBF_ERR_INVALID, "surface too large: more than 2^28 triangles");
   const size_t slots = surface_hash_slots(cap);
   const size_t need = slots * (sizeof(unsigned long long) + sizeof(float4)) + 6 * sizeof(uint32_t) * cap + 512;
@@ -1041,8 +1069,10 @@ pbf_status Handle::surface_emit(const SurfGrid& g, double isolevel, float* xyz, 
   hs.vslot = reinterpret_cast<uint32_t*>(hs.nslot + slots);
   hs.ulist = hs.vslot + 3 * static_cast<size_t>(cap);
   hs.ucount = hs.ulist + 3 * static_cast<size_t>(cap);
-  return cuda(launch_surface_emit(b, dp, cur, g, static_cast<float>(isolevel), surf_table_dev, field, first, xyz, nrm,
-                                  cap, hs, stream),
+  return cuda(launch_surface_emit(b, dp, cur, g, static_cast<float>(isolevel), surf_table_dev,
+                                  reinterpret_cast<const float*>(base),
+                                  reinterpret_cast<const uint32_t*>(base + w.first),
+                                  reinterpret_cast<const uint32_t*>(base + w.tile), xyz, nrm, cap, hs, stream),
               "surface emit");
 }
 
@@ -1063,16 +1093,16 @@ pbf_status pbf_surface(pbf_handle* hh, double isolevel, double step, const doubl
   *count = total;
   const size_t m = std::min(static_cast<size_t>(total), cap);
   if (m == 0) return PBF_OK;
-  float* dev = nullptr;
-  st = h->cuda(cudaMalloc(&dev, sizeof(float) * 18 * m), "cudaMalloc(surface)");
+  if (m > (size_t(1) << 28)) return h->fail(PBF_ERR_INVALID, "surface too large: more than 2^28 triangles");
+  st = h->ensure_surface_out(sizeof(float) * 18 * m);
   if (st != PBF_OK) return st;
+  float* dev = h->surf_out;
   st = h->surface_emit(g, isolevel, dev, dev + 9 * m, static_cast<uint32_t>(m));
   if (st == PBF_OK)
     st = h->cuda(cudaMemcpyAsync(xyz, dev, sizeof(float) * 9 * m, cudaMemcpyDeviceToHost, h->stream), "D2H");
   if (st == PBF_OK)
     st = h->cuda(cudaMemcpyAsync(nrm, dev + 9 * m, sizeof(float) * 9 * m, cudaMemcpyDeviceToHost, h->stream), "D2H");
   if (st == PBF_OK) st = h->cuda(cudaStreamSynchronize(h->stream), "sync");
-  cudaFree(dev);
   return st;
 }
 

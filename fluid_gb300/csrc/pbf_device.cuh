@@ -759,9 +759,9 @@ __device__ __forceinline__ bool spiky_s(float r2, float h, float* s) {
 // trimmed in x to the cells that reach [x - w, x + w], w = sqrt(h^2 - d_yz^2), with a
 // margin of 1e-3 cell: only particles that add nothing are left out, so the sum (same
 // rows, same slot order) is the same.
-__device__ __forceinline__ float density_at_point(const float3 p, const float4* __restrict__ pos,
-                                                  const uint32_t* __restrict__ cell_start, const SceneDesc& sc,
-                                                  const DevParams& P) {
+__device__ __forceinline__ float density_sum_at(const float3 p, const float4* __restrict__ pos,
+                                                const uint32_t* __restrict__ cell_start, const SceneDesc& sc,
+                                                const DevParams& P) {
   const CellCoord cc = cell_of(p, sc, P.inv_cell);
   const float m = 1e-3f;
   const float reach = sqrtf(P.h2) * P.inv_cell + m;
@@ -793,7 +793,61 @@ __device__ __forceinline__ float density_at_point(const float3 p, const float4* 
       }
     }
   }
-  return P.poly6_c * qsum;
+  return qsum;
+}
+__device__ __forceinline__ float density_at_point(const float3 p, const float4* __restrict__ pos,
+                                                  const uint32_t* __restrict__ cell_start, const SceneDesc& sc,
+                                                  const DevParams& P) {
+  return P.poly6_c * density_sum_at(p, pos, cell_start, sc, P);
+}
+
+// Whether p's cell needs no clamping to the grid.
+__device__ __forceinline__ bool in_grid(const float3 p, const SceneDesc& sc, float inv_cell) {
+  const float u = (p.x - sc.origin[0]) * inv_cell, v = (p.y - sc.origin[1]) * inv_cell,
+              w = (p.z - sc.origin[2]) * inv_cell;
+  return u >= 0.f && v >= 0.f && w >= 0.f && u < static_cast<float>(sc.dim[0]) &&
+         v < static_cast<float>(sc.dim[1]) && w < static_cast<float>(sc.dim[2]);
+}
+
+// density_at_point for lanes whose points lie close together, in the grid and in [lo, hi] (the same
+// for these lanes): they walk the rows around the whole box together, so a candidate is one
+// broadcast load for all of them. Every particle within h of a point lies in the walk, the others
+// add zero, and the order is density_at_point's: the same bits. Returns the sum without its factor
+// poly6_c, as density_sum_at does.
+__device__ __forceinline__ float density_together(const float3 p, const float3 lo, const float3 hi,
+                                                  const float4* __restrict__ pos,
+                                                  const uint32_t* __restrict__ cell_start, const SceneDesc& sc,
+                                                  const DevParams& P) {
+  const float m = 1e-3f;
+  const float reach = sqrtf(P.h2) * P.inv_cell + m;
+  const float reach2 = reach * reach;
+  const float x0 = (lo.x - sc.origin[0]) * P.inv_cell, x1 = (hi.x - sc.origin[0]) * P.inv_cell;
+  const float y0 = (lo.y - sc.origin[1]) * P.inv_cell, y1 = (hi.y - sc.origin[1]) * P.inv_cell;
+  const float z0 = (lo.z - sc.origin[2]) * P.inv_cell, z1 = (hi.z - sc.origin[2]) * P.inv_cell;
+  const int zb = min(static_cast<int>(floorf(z1)) + 1, sc.dim[2] - 1);
+  const int yb = min(static_cast<int>(floorf(y1)) + 1, sc.dim[1] - 1);
+  const int xl = max(static_cast<int>(floorf(x0)) - 1, 0), xr = min(static_cast<int>(floorf(x1)) + 1, sc.dim[0] - 1);
+  float sum = 0.f;
+  for (int z = max(static_cast<int>(floorf(z0)) - 1, 0); z <= zb; ++z)
+    for (int y = max(static_cast<int>(floorf(y0)) - 1, 0); y <= yb; ++y) {
+      const float dy = fmaxf(fmaxf(static_cast<float>(y) - y1, y0 - static_cast<float>(y + 1)) - m, 0.f);
+      const float dz = fmaxf(fmaxf(static_cast<float>(z) - z1, z0 - static_cast<float>(z + 1)) - m, 0.f);
+      const float w2 = reach2 - (dy * dy + dz * dz);
+      if (w2 < 0.f) continue;
+      const float w = sqrtf(w2);
+      const int xa = max(static_cast<int>(floorf(x0 - w)), xl), xb = min(static_cast<int>(floorf(x1 + w)), xr);
+      if (xa > xb) continue;
+      const uint32_t row = sc.cell_off + static_cast<uint32_t>((z * sc.dim[1] + y) * sc.dim[0]);
+      const uint32_t e = __ldg(&cell_start[row + xb + 1]);
+#pragma unroll 4
+      for (uint32_t j = __ldg(&cell_start[row + xa]); j < e; ++j) {
+        const float4 xj = __ldg(&pos[j]);
+        const float dx = xj.x - p.x, ey = xj.y - p.y, ez = xj.z - p.z;
+        const float t = fmaxf(P.h2 - __fmaf_rn(ez, ez, __fmaf_rn(dx, dx, __fmul_rn(ey, ey))), 0.f);
+        sum = __fmaf_rn(__fmul_rn(t, t), t, sum);
+      }
+    }
+  return sum;
 }
 
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }

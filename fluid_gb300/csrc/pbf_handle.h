@@ -61,6 +61,8 @@ struct Handle {
   SurfTable* surf_table_dev = nullptr;  // marching-cubes table (first pbf_surface)
   void* surf_hash = nullptr;            // grow-only scratch of the surface's vertex-normal table
   size_t surf_hash_bytes = 0;
+  float* surf_out = nullptr;            // grow-only: the triangles of pbf_surface before their copy to the host
+  size_t surf_out_bytes = 0;
   float4* mesh_dev = nullptr;           // collider triangles and their hierarchy (pbf_set_collider_mesh)
   float4* sph_dev = nullptr;            // collider spheres (pbf_set_collider_spheres)
   RenderState render;                   // path tracer (pbf_render_set_scene, pbf_render)
@@ -72,6 +74,9 @@ struct Handle {
   pbf_status alloc_all();
   void free_all();
   pbf_status ensure_scratch(size_t bytes);
+  pbf_status ensure_surface_out(size_t bytes);
+  struct SurfScratch;
+  SurfScratch surface_scratch(const SurfGrid& g) const;
   pbf_status ensure_tape();
   void free_tape();
   pbf_status surface_count(double isolevel, double step, const double* lo, const double* hi, SurfGrid* g,

@@ -257,11 +257,13 @@ uint32_t exclusive_scan_tiles(uint32_t m);
 cudaError_t launch_density_at(const Buffers& b, const DevParams& p, int cur, size_t m,
                               const float* pts, float* out, cudaStream_t s);
 // ---- surface (pbf_surface.cu), on the cell-sorted state in buffers cur ----
-// field: (nc+1)^3 corner values; count: per-cube triangle counts; first: their exclusive
-// scan (first[cubes] = total); tile_sums: exclusive_scan_tiles(cubes) entries.
+// any: a byte per grid cell of the handle; field: (nc+1)^3 corner values, z fastest; first: per
+// cube, the triangles of the cubes before it in its tile; tile: the exclusive scan of the tiles'
+// triangles, surface_tiles(cubes) entries and the total.
+uint32_t surface_tiles(uint32_t cubes);
 cudaError_t launch_surface_count(const Buffers& b, const DevParams& p, int cur, const SurfGrid& g, float iso,
-                                 const SurfTable* tab, float* field, uint32_t* count, uint32_t* first,
-                                 uint32_t* tile_sums, cudaStream_t s);
+                                 const SurfTable* tab, uint8_t* any, float* field, uint32_t* first, uint32_t* tile,
+                                 cudaStream_t s);
 // Scratch of launch_surface_emit for cap triangles: keys and nslot hold
 // surface_hash_slots(cap) entries, vslot and ulist 3 * cap, ucount one.
 struct SurfHash {
@@ -273,7 +275,8 @@ uint32_t surface_hash_slots(uint32_t triangles);
 // Triangles with index < cap (cap at most the total of the counts): 9 floats of vertices
 // and 9 of vertex normals each. Each vertex normal is evaluated once per grid edge.
 cudaError_t launch_surface_emit(const Buffers& b, const DevParams& p, int cur, const SurfGrid& g, float iso,
-                                const SurfTable* tab, const float* field, const uint32_t* first, float* xyz,
-                                float* nrm, uint32_t cap, const SurfHash& hs, cudaStream_t s);
+                                const SurfTable* tab, const float* field, const uint32_t* first,
+                                const uint32_t* tile, float* xyz, float* nrm, uint32_t cap, const SurfHash& hs,
+                                cudaStream_t s);
 
 }  // namespace pbf
