@@ -340,14 +340,20 @@ class Simulator:
         lo_a = None if lo is None else np.ascontiguousarray(lo, dtype=np.float64)
         hi_a = None if hi is None else np.ascontiguousarray(hi, dtype=np.float64)
         count = ctypes.c_size_t(0)
-        self._check(lib().pbf_surface(self._h, iso, step, _ptr(lo_a), _ptr(hi_a), None, None, 0,
-                                      ctypes.byref(count)))
-        t = count.value
-        xyz = np.zeros((max(t, 1), 3, 3), dtype=np.float32)
-        nrm = np.zeros((max(t, 1), 3, 3), dtype=np.float32)
-        self._check(lib().pbf_surface(self._h, iso, step, _ptr(lo_a), _ptr(hi_a), _ptr(xyz), _ptr(nrm), t,
-                                      ctypes.byref(count)))
-        return xyz[:t], nrm[:t]
+        # One call when the triangles fit the room made for them (a surface grows with the square of
+        # the cubes across the particles' extent; pages that stay untouched cost nothing), else a
+        # second one with the room the first reported.
+        room = 4096 + int(48.0 * (0.5 * self.params.h / step) ** 2 * self.n ** (2.0 / 3.0)) if step > 0 else 4096
+        room = min(room, 1 << 26)
+        while True:
+            xyz = np.empty((room, 3, 3), dtype=np.float32)
+            nrm = np.empty((room, 3, 3), dtype=np.float32)
+            self._check(lib().pbf_surface(self._h, iso, step, _ptr(lo_a), _ptr(hi_a), _ptr(xyz), _ptr(nrm), room,
+                                          ctypes.byref(count)))
+            t = count.value
+            if t <= room:
+                return xyz[:t], nrm[:t]
+            room = t
 
     def set_render_scene(self, scene):
         """The scene the fluid is rendered in (a fluid_gb300.render.RenderScene)."""
