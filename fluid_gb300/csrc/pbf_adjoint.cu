@@ -78,6 +78,7 @@ __global__ void k_adj_in(const uint32_t* __restrict__ id, const float* __restric
                          const float4* __restrict__ omega, float4* __restrict__ gxs, float4* __restrict__ gvo,
                          float4* __restrict__ eb, float4* __restrict__ wb, float* __restrict__ r0, DevParams P,
                          float dt, int n) {
+  chain_begin();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const uint32_t o = id[s];
@@ -113,6 +114,7 @@ __global__ void __launch_bounds__(BLOCK) k_adj_vort_b(const float4* __restrict__
                                                       const uint32_t* __restrict__ words,
                                                       const float4* __restrict__ eb, float4* __restrict__ wb,
                                                       float4* __restrict__ gxs, DevParams P, int n) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 xi = xs[i];  // w: |omega_i|
@@ -198,6 +200,7 @@ __global__ void __launch_bounds__(BLOCK) k_adj_xsph(const float4* __restrict__ x
                                                     const float4* __restrict__ gvo, const float4* __restrict__ wb,
                                                     Finish F, DevParams P, float dt, float inv_dt, int last,
                                                     int n) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 xi = xs[i];
@@ -236,6 +239,7 @@ __global__ void __launch_bounds__(BLOCK) k_adj_lambda(const float4* __restrict__
                                                       const uint32_t* __restrict__ words,
                                                       const float4* __restrict__ pl, float4* __restrict__ gr,
                                                       float* __restrict__ r0, DevParams P, int n) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 xi = xs[i];
@@ -272,6 +276,7 @@ __global__ void __launch_bounds__(BLOCK) k_adj_pos(const float4* __restrict__ xs
                                                    const uint32_t* __restrict__ words,
                                                    const float4* __restrict__ pl, const float4* __restrict__ gr,
                                                    Finish F, DevParams P, float dt, int next, int n) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 xi = xs[i];
@@ -321,6 +326,7 @@ __global__ void __launch_bounds__(BLOCK) k_adj_pos(const float4* __restrict__ xs
 // rest-density adjoint: fixed-shape two-level sum (deterministic)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_adj_r0_part(const float* __restrict__ r0, double* __restrict__ part, int n) {
+  chain_begin();
   double acc = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) acc += r0[i];
   __shared__ double sh[256];
@@ -335,6 +341,7 @@ __global__ void __launch_bounds__(256) k_adj_r0_part(const float* __restrict__ r
 
 __global__ void __launch_bounds__(kAdjReduceBlocks) k_adj_r0_final(const double* __restrict__ part,
                                                                    double* __restrict__ out) {
+  chain_begin();
   __shared__ double sh[kAdjReduceBlocks];
   sh[threadIdx.x] = part[threadIdx.x];
   __syncthreads();
@@ -373,32 +380,32 @@ cudaError_t launch_adjoint(const Buffers& b, const DevParams& P, const Tuning& t
   F.gx_in = gx_in;
   F.gv_in = gv_in;
   F.n = b.n;
-  k_adj_in<<<blocks_for(n, 256), 256, 0, s>>>(b.id[B], gx_out, gv_out, tp.eta, b.omega, tp.gxs, tp.gvo, tp.eb,
-                                              tp.wb, tp.r0, P, dt, n);
+  chain_launch(k_adj_in, blocks_for(n, 256), 256, 0, s, b.id[B], gx_out, gv_out, tp.eta, b.omega, tp.gxs, tp.gvo, tp.eb,
+               tp.wb, tp.r0, P, dt, n);
   PBF_BLOCK_SWITCH(t.block_solve,
-                   k_adj_vort_b<BLOCK><<<blocks_for(n, BLOCK), BLOCK, 0, s>>>(
-                       fin, b.omega, b.nbr_hdr, b.nbr_w, tp.eb, tp.wb, tp.gxs, P, n));
+                   chain_launch(k_adj_vort_b<BLOCK>, blocks_for(n, BLOCK), BLOCK, 0, s, fin, b.omega, b.nbr_hdr,
+                                b.nbr_w, tp.eb, tp.wb, tp.gxs, P, n));
   PBF_BLOCK_SWITCH(t.block_solve,
-                   k_adj_xsph<BLOCK><<<blocks_for(n, BLOCK), BLOCK, 0, s>>>(
-                       fin, b.disp[1], b.nbr_hdr, b.nbr_w, tp.gvo, tp.wb, F, P, dt, inv_dt, I - 1, n));
+                   chain_launch(k_adj_xsph<BLOCK>, blocks_for(n, BLOCK), BLOCK, 0, s, fin, b.disp[1], b.nbr_hdr,
+                                b.nbr_w, tp.gvo, tp.wb, F, P, dt, inv_dt, I - 1, n));
   for (int k = I - 1; k >= 0; --k) {
     const float4* xk = tp.xs + static_cast<size_t>(k) * b.n;
     const float4* plk = tp.pl[k & 1];
     PBF_BLOCK_SWITCH(t.block_solve,
-                     k_adj_lambda<BLOCK><<<blocks_for(n, BLOCK), BLOCK, 0, s>>>(
-                         xk, b.nbr_hdr, b.nbr_w, plk, tp.gr, tp.r0, P, n));
+                     chain_launch(k_adj_lambda<BLOCK>, blocks_for(n, BLOCK), BLOCK, 0, s, xk, b.nbr_hdr, b.nbr_w, plk,
+                                  tp.gr, tp.r0, P, n));
     if (P.scorr_n == 4) {
       PBF_BLOCK_SWITCH(t.block_solve,
-                       (k_adj_pos<BLOCK, true><<<blocks_for(n, BLOCK), BLOCK, 0, s>>>(
-                           xk, b.nbr_hdr, b.nbr_w, plk, tp.gr, F, P, dt, k - 1, n)));
+                       (chain_launch((k_adj_pos<BLOCK, true>), blocks_for(n, BLOCK), BLOCK, 0, s, xk, b.nbr_hdr,
+                                     b.nbr_w, plk, tp.gr, F, P, dt, k - 1, n)));
     } else {
       PBF_BLOCK_SWITCH(t.block_solve,
-                       (k_adj_pos<BLOCK, false><<<blocks_for(n, BLOCK), BLOCK, 0, s>>>(
-                           xk, b.nbr_hdr, b.nbr_w, plk, tp.gr, F, P, dt, k - 1, n)));
+                       (chain_launch((k_adj_pos<BLOCK, false>), blocks_for(n, BLOCK), BLOCK, 0, s, xk, b.nbr_hdr,
+                                     b.nbr_w, plk, tp.gr, F, P, dt, k - 1, n)));
     }
   }
-  k_adj_r0_part<<<kAdjReduceBlocks, 256, 0, s>>>(tp.r0, tp.r0_part, n);
-  k_adj_r0_final<<<1, kAdjReduceBlocks, 0, s>>>(tp.r0_part, g_rho0);
+  chain_launch(k_adj_r0_part, kAdjReduceBlocks, 256, 0, s, tp.r0, tp.r0_part, n);
+  chain_launch(k_adj_r0_final, 1, kAdjReduceBlocks, 0, s, tp.r0_part, g_rho0);
   return cudaGetLastError();
 }
 

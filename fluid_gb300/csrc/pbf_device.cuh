@@ -9,6 +9,30 @@
 
 namespace pbf {
 
+// Programmatic dependent launch. Every kernel of the step's chains begins with chain_begin(): it
+// waits until the kernel before has finished and its writes are visible. All threads call it before
+// anything else, so a kernel is done only after the one before it. What it hides is the launch
+// itself: 33k particles with a mesh 258 -> 219 us a step, the adjoint of 262k 767 -> 711. A kernel
+// lets the next one's blocks in only when its own are done: let in earlier (launch_dependents at
+// the start of a kernel), they hold the places of blocks that could work (1M: 806 -> 1,236 us).
+__device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Launches such a kernel behind the one before it in the stream.
+template <typename... Params, typename... Args>
+inline cudaError_t chain_launch(void (*kernel)(Params...), size_t grid, size_t block, size_t smem, cudaStream_t s,
+                                Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(block));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 __device__ __forceinline__ float3 f3(const float4& a) { return make_float3(a.x, a.y, a.z); }
 __device__ __forceinline__ float3 operator+(float3 a, float3 b) { return make_float3(a.x + b.x, a.y + b.y, a.z + b.z); }
 __device__ __forceinline__ float3 operator-(float3 a, float3 b) { return make_float3(a.x - b.x, a.y - b.y, a.z - b.z); }

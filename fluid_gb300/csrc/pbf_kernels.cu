@@ -49,6 +49,7 @@ __global__ void k_predict(const float4* __restrict__ pos, const float4* __restri
                           uint32_t* __restrict__ cell_count,
                           const SceneDesc* __restrict__ scenes, DevParams P, float dt, int move,
                           int n) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = i < n;
   uint32_t key = 0xffffffffu;
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t* __restric
                                                               uint32_t* __restrict__ tile_sum,
                                                               uint32_t m, uint32_t* __restrict__ ticket,
                                                               uint32_t* __restrict__ zero_word) {
+  chain_begin();
   const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
   uint32_t s = 0;
@@ -169,12 +171,14 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(uint32_t* __restric
 __global__ void __launch_bounds__(1024) k_scan_sums(uint32_t* __restrict__ tile_sum, uint32_t tiles,
                                                      uint32_t* __restrict__ start, uint32_t m,
                                                      uint32_t* __restrict__ zero_word) {
+  chain_begin();
   scan_tile_sums(tile_sum, tiles, start, m, zero_word);
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_add(uint32_t* __restrict__ start,
                                                             const uint32_t* __restrict__ tile_sum,
                                                             uint32_t m) {
+  chain_begin();
   const uint32_t add = tile_sum[blockIdx.x];
   const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
 #pragma unroll
@@ -187,6 +191,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_add(uint32_t* __restrict_
 // ---------------------------------------------------------------------------
 __global__ void k_scatter(const uint32_t* __restrict__ key, const uint32_t* __restrict__ rank,
                           const uint32_t* __restrict__ cell_start, uint32_t* __restrict__ perm, int n) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) perm[cell_start[key[i]] + rank[i]] = static_cast<uint32_t>(i);
 }
@@ -212,6 +217,7 @@ __global__ void k_cellrank(const uint32_t* __restrict__ cell_start, const uint32
                            const uint32_t* __restrict__ key, const uint32_t* __restrict__ xkey,
                            const uint32_t* __restrict__ id, uint32_t* __restrict__ perm,
                            uint32_t* __restrict__ big_cells, uint32_t* __restrict__ big_count, int n) {
+  chain_begin();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const uint32_t v = atomic_order[s];
@@ -238,6 +244,7 @@ __global__ void __launch_bounds__(kBigSortThreads) k_cellsort_big(const uint32_t
                                                                  const uint32_t* __restrict__ id,
                                                                  const uint32_t* __restrict__ big_cells,
                                                                  const uint32_t* __restrict__ big_count) {
+  chain_begin();
   __shared__ uint32_t slot[kMaxSortedCell];
   __shared__ uint32_t khi[kMaxSortedCell];
   __shared__ uint32_t klo[kMaxSortedCell];
@@ -270,6 +277,7 @@ __global__ void k_gather(const uint32_t* __restrict__ perm, const float4* __rest
                          const uint32_t* __restrict__ id_a, float4* __restrict__ pos_b,
                          float4* __restrict__ disp_b, float4* __restrict__ xs_b,
                          float4* __restrict__ vel_b, uint32_t* __restrict__ id_b, int n) {
+  chain_begin();
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const uint32_t i = perm[s];
@@ -301,6 +309,7 @@ __global__ void __launch_bounds__(BLOCK, 1152 / BLOCK) k_nbr_build(const float4*
                                                      const SceneDesc* __restrict__ scenes,
                                                      uint4* __restrict__ hdr, uint32_t* __restrict__ words,
                                                      unsigned* __restrict__ err, DevParams P, float one, int n) {
+  chain_begin();
   extern __shared__ uint4 nbr_smem[];
   nbr_build_warp<true>(reinterpret_cast<NbrWarp*>(nbr_smem)[threadIdx.x >> 5],
                        static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x), xs, pos, cell_start, scenes, hdr,
@@ -317,6 +326,7 @@ __global__ void __launch_bounds__(BLOCK) k_lambda(float4* xs, const uint4* __res
                                                   const uint32_t* __restrict__ words,
                                                   float* __restrict__ rho_iter0,
                                                   DevParams P, int n) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 xi = xs[i];
@@ -344,6 +354,7 @@ __global__ void __launch_bounds__(BLOCK) k_deltap(const float4* __restrict__ xs,
                                                   const SceneDesc* __restrict__ scenes,
                                                   float4* __restrict__ disp, float4* __restrict__ xs_next,
                                                   float4* __restrict__ dp_rec, DevParams P, int n) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 xi = xs[i];
@@ -377,6 +388,7 @@ __global__ void __launch_bounds__(BLOCK) k_xsph(float4* xs, const float4* __rest
                                                 float4* __restrict__ vel_out, float4* __restrict__ omega,
                                                 float* __restrict__ rho_out, DevParams P, float inv_dt,
                                                 int n) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 xi = xs[i];
@@ -401,6 +413,7 @@ __global__ void __launch_bounds__(BLOCK) k_vort(const float4* __restrict__ xs,
                                                 const uint32_t* __restrict__ words,
                                                 float4* __restrict__ vel, unsigned* __restrict__ err,
                                                 float4* __restrict__ eta_rec, DevParams P, float dt, int n) {
+  chain_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float4 xi = xs[i];
@@ -500,6 +513,7 @@ template <bool JOIN>
 __global__ void __launch_bounds__(256) k_stats(const float* __restrict__ rho, const float* __restrict__ rho0,
                                                const uint4* __restrict__ hdr, DevStats* part,
                                                DevStats* __restrict__ st, unsigned* ticket, float inv_rho0, int n) {
+  chain_begin();
   StatsAcc s{0.f, 0.f, 0.f, 0.f, 0xffffffffu, 0u, 0u, 0u};
   const int n4 = n / 4;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n4; k += gridDim.x * blockDim.x) {
@@ -547,6 +561,7 @@ __global__ void __launch_bounds__(256) k_stats(const float* __restrict__ rho, co
 
 __global__ void __launch_bounds__(kStatsBlocks) k_stats_final(const DevStats* __restrict__ part,
                                                               DevStats* __restrict__ st) {
+  chain_begin();
   DevStats a = part[threadIdx.x];
   a = stats_block_reduce(a);
   if (threadIdx.x == 0) *st = a;
@@ -674,7 +689,7 @@ __global__ void k_density_at(const float4* __restrict__ pos, const uint32_t* __r
 inline unsigned blocks_for(size_t n, int block) { return static_cast<unsigned>((n + block - 1) / block); }
 
 // Launches neighbour kernel KERN (a template-id, parenthesised) over n particles, BLOCK threads a block.
-#define PBF_PASS_LAUNCH(KERN, ...) KERN<<<blocks_for(n, BLOCK), BLOCK, 0, s>>>(__VA_ARGS__)
+#define PBF_PASS_LAUNCH(KERN, ...) chain_launch(KERN, blocks_for(n, BLOCK), BLOCK, 0, s, __VA_ARGS__)
 
 // Instantiates a neighbour pass for the tuned gather depth (D = 4 or 8 neighbour loads in
 // flight per thread) and list-load policy (ST: streaming). Neither changes the order in
@@ -699,16 +714,16 @@ cudaError_t launch_nbr_build(const Buffers& b, const DevParams& P, const float4*
                                          static_cast<int>(bytes));
     if (e != cudaSuccess) return e;
   }
-  k_nbr_build<BLOCK><<<blocks_for(n, BLOCK), BLOCK, bytes, s>>>(xs, pos, b.cell_start, b.scenes, b.nbr_hdr, b.nbr_w,
-                                                               b.err, P, 1.0f, n);
+  chain_launch(k_nbr_build<BLOCK>, blocks_for(n, BLOCK), BLOCK, bytes, s, xs, pos, b.cell_start, b.scenes, b.nbr_hdr,
+               b.nbr_w, b.err, P, 1.0f, n);
   return cudaGetLastError();
 }
 
 void launch_stats(const Buffers& b, const DevParams& P, bool join, cudaStream_t s) {
   auto kern = join ? k_stats<true> : k_stats<false>;
-  kern<<<kStatsBlocks, 256, 0, s>>>(b.rho, b.rho_iter0, b.nbr_hdr, b.stats_part, b.stats, b.grid_bar + 2, P.inv_rho0,
-                                    static_cast<int>(b.n));
-  if (!join) k_stats_final<<<1, kStatsBlocks, 0, s>>>(b.stats_part, b.stats);
+  chain_launch(kern, kStatsBlocks, 256, 0, s, b.rho, b.rho_iter0, b.nbr_hdr, b.stats_part, b.stats, b.grid_bar + 2,
+               P.inv_rho0, static_cast<int>(b.n));
+  if (!join) chain_launch(k_stats_final, 1, kStatsBlocks, 0, s, b.stats_part, b.stats);
 }
 
 // One delta-p pass (B = the buffer index holding this step's cell-ordered x and delta).
@@ -728,7 +743,8 @@ void launch_deltap(const Tuning& t, const Buffers& b, int B, float4* xcur, float
                                                    b.nbr_hdr, b.nbr_w, b.scenes, b.disp[1], xnext, dprec, P, n)));
 }
 
-// Shared front half of a step and of a resort: keys, counts, scan, slots.
+// Shared front half of a step and of a resort: keys, counts, scan, slots. Its first kernel is launched
+// plainly: what comes before it in the stream may be a wait for another stream's event.
 cudaError_t sort_into_cells(const Buffers& b, const DevParams& P, const Tuning& t, int cur, float dt,
                             bool move, cudaStream_t s, PhaseMarks* mk = nullptr, bool rec = false) {
   const int n = static_cast<int>(b.n);
@@ -742,15 +758,16 @@ cudaError_t sort_into_cells(const Buffers& b, const DevParams& P, const Tuning& 
   if (mk) mk->mark(kPhasePredict, s);
   const uint32_t tiles = (m + kScanTile - 1) / kScanTile;
   // scan_tmp holds the tile sums and, after them, the ticket of k_scan_tiles' last block
-  k_scan_tiles<true><<<tiles, kScanThreads, 0, s>>>(b.cell_count, b.cell_start, b.scan_tmp, m, b.scan_tmp + tiles,
-                                               b.big_count);
-  k_scan_add<<<tiles, kScanThreads, 0, s>>>(b.cell_start, b.scan_tmp, m);
+  chain_launch(k_scan_tiles<true>, tiles, kScanThreads, 0, s, b.cell_count, b.cell_start, b.scan_tmp, m,
+               b.scan_tmp + tiles, b.big_count);
+  chain_launch(k_scan_add, tiles, kScanThreads, 0, s, b.cell_start, b.scan_tmp, m);
   if (mk) mk->mark(kPhaseScan, s);
-  k_scatter<<<blocks_for(n, t.block_misc), t.block_misc, 0, s>>>(b.key, b.rank, b.cell_start, b.perm_atomic, n);
-  k_cellrank<<<blocks_for(n, t.block_misc), t.block_misc, 0, s>>>(b.cell_start, b.perm_atomic, b.key, b.xkey,
-                                                                   b.id[cur], b.perm, b.big_cells, b.big_count, n);
-  k_cellsort_big<<<kBigSortBlocks, kBigSortThreads, 0, s>>>(b.cell_start, b.perm, b.xkey, b.id[cur], b.big_cells,
-                                                             b.big_count);
+  chain_launch(k_scatter, blocks_for(n, t.block_misc), t.block_misc, 0, s, b.key, b.rank, b.cell_start, b.perm_atomic,
+               n);
+  chain_launch(k_cellrank, blocks_for(n, t.block_misc), t.block_misc, 0, s, b.cell_start, b.perm_atomic, b.key, b.xkey,
+               b.id[cur], b.perm, b.big_cells, b.big_count, n);
+  chain_launch(k_cellsort_big, kBigSortBlocks, kBigSortThreads, 0, s, b.cell_start, b.perm, b.xkey, b.id[cur],
+               b.big_cells, b.big_count);
   if (mk) mk->mark(kPhaseSort, s);
   return cudaGetLastError();
 }
@@ -774,9 +791,8 @@ cudaError_t launch_step(const Buffers& b, const DevParams& P, const Tuning& t, i
   cudaError_t e = sort_into_cells(b, P, t, A, dt, true, s, mk, rec);
   if (e != cudaSuccess) return e;
   float4* xs0 = rec ? tape->xs : b.xs[0];
-  k_gather<<<blocks_for(n, t.block_misc), t.block_misc, 0, s>>>(
-      b.perm, b.pos[A], b.disp[0], rec ? b.vel[A] : nullptr, b.id[A], b.pos[B], b.disp[1], xs0,
-      rec ? tape->v : nullptr, b.id[B], n);
+  chain_launch(k_gather, blocks_for(n, t.block_misc), t.block_misc, 0, s, b.perm, b.pos[A], b.disp[0],
+               rec ? b.vel[A] : nullptr, b.id[A], b.pos[B], b.disp[1], xs0, rec ? tape->v : nullptr, b.id[B], n);
   if (rec) {
     e = cudaMemcpyAsync(tape->x, b.pos[B], sizeof(float4) * b.n, cudaMemcpyDeviceToDevice, s);
     if (e != cudaSuccess) return e;
@@ -838,9 +854,8 @@ cudaError_t launch_resort(const Buffers& b, const DevParams& P, const Tuning& t,
   if (n == 0) return cudaSuccess;
   cudaError_t e = sort_into_cells(b, P, t, cur, 0.f, false, s);
   if (e != cudaSuccess) return e;
-  k_gather<<<blocks_for(n, t.block_misc), t.block_misc, 0, s>>>(
-      b.perm, b.pos[cur], nullptr, b.vel[cur], b.id[cur], b.pos[1 - cur], nullptr, nullptr, b.vel[1 - cur],
-      b.id[1 - cur], n);
+  chain_launch(k_gather, blocks_for(n, t.block_misc), t.block_misc, 0, s, b.perm, b.pos[cur], nullptr, b.vel[cur],
+               b.id[cur], b.pos[1 - cur], nullptr, nullptr, b.vel[1 - cur], b.id[1 - cur], n);
   return cudaGetLastError();
 }
 
@@ -899,9 +914,10 @@ cudaError_t launch_neighbor_ids(const Buffers& b, int cur, const uint32_t* offse
 cudaError_t launch_exclusive_scan(const uint32_t* count, uint32_t* start, uint32_t* tile_sums, uint32_t m,
                                   cudaStream_t s) {
   const uint32_t tiles = (m + kScanTile - 1) / kScanTile;
-  k_scan_tiles<false><<<tiles, kScanThreads, 0, s>>>(const_cast<uint32_t*>(count), start, tile_sums, m, nullptr, nullptr);
-  k_scan_sums<<<1, 1024, 0, s>>>(tile_sums, tiles, start, m, nullptr);
-  k_scan_add<<<tiles, kScanThreads, 0, s>>>(start, tile_sums, m);
+  chain_launch(k_scan_tiles<false>, tiles, kScanThreads, 0, s, const_cast<uint32_t*>(count), start, tile_sums, m,
+               nullptr, nullptr);
+  chain_launch(k_scan_sums, 1, 1024, 0, s, tile_sums, tiles, start, m, nullptr);
+  chain_launch(k_scan_add, tiles, kScanThreads, 0, s, start, tile_sums, m);
   return cudaGetLastError();
 }
 

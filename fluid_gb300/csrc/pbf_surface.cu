@@ -168,6 +168,7 @@ __device__ __forceinline__ float3 corner_point(const SurfGrid& g, int i, int j, 
 // see none (3 of 4 over a box a quarter full), and leave k_surf_density after one byte.
 __global__ void k_surf_cells(const uint32_t* __restrict__ cell_start, const SceneDesc* __restrict__ scenes,
                              uint8_t* __restrict__ any, uint32_t m) {
+  chain_begin();
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m) return;
   const SceneDesc& sc = scenes[0];
@@ -193,6 +194,7 @@ __global__ void __launch_bounds__(128) k_surf_density(const float4* __restrict__
                                                       const SceneDesc* __restrict__ scenes,
                                                       const uint8_t* __restrict__ any, SurfGrid g,
                                                       float* __restrict__ field, DevParams P) {
+  chain_begin();
   const int nx = g.nc[0] + 1, ny = g.nc[1] + 1, nz = g.nc[2] + 1;
   const int lane = static_cast<int>(lane_id()), warp = static_cast<int>(threadIdx.x >> 5);
   const int bx = (nx + 1) / 2, by = (ny + 7) / 8;
@@ -252,6 +254,7 @@ __global__ void __launch_bounds__(kCubeTile / 4) k_surf_count(const float* __res
                                                               const SurfTable* __restrict__ tab, SurfGrid g,
                                                               float iso, uint32_t* __restrict__ first,
                                                               uint32_t* __restrict__ tile, uint32_t ncubes) {
+  chain_begin();
   __shared__ uint8_t ntri[256];
   __shared__ uint32_t sums[kCubeTile / 128];
   for (unsigned k = threadIdx.x; k < 256; k += blockDim.x) ntri[k] = tab->ntri[k];
@@ -284,6 +287,7 @@ __global__ void __launch_bounds__(kCubeTile / 4) k_surf_count(const float* __res
 
 // Exclusive scan of the tiles' sums in place; tile[tiles] = the total.
 __global__ void __launch_bounds__(1024) k_surf_tiles(uint32_t* __restrict__ tile, uint32_t tiles) {
+  chain_begin();
   __shared__ uint32_t sums[32];
   uint32_t carry = 0;
   for (uint32_t b = 0; b < tiles; b += 4 * blockDim.x) {
@@ -387,6 +391,7 @@ __global__ void k_surf_vertices(const float* __restrict__ field, const SurfTable
                                 uint32_t count, uint32_t ncubes, unsigned long long* keys, uint32_t cap_mask,
                                 uint32_t* __restrict__ vslot, uint32_t* __restrict__ ulist, uint32_t* ucount,
                                 float* __restrict__ xyz) {
+  chain_begin();
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= 3u * count) return;
   const TriVertex r = tri_vertex(field, tab, g, iso, first, tile, ncubes, tid / 3u, static_cast<int>(tid % 3u));
@@ -434,6 +439,7 @@ __global__ void __launch_bounds__(128) k_surf_vnormals(const float* __restrict__
                                                        float4* __restrict__ nslot, const float4* __restrict__ pos,
                                                        const uint32_t* __restrict__ cell_start,
                                                        const SceneDesc* __restrict__ scenes, DevParams P) {
+  chain_begin();
   const uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   if ((u & ~3u) >= *ucount) return;  // none of the warp's 4 slots
   const int lane = static_cast<int>(lane_id());
@@ -472,6 +478,7 @@ __global__ void __launch_bounds__(128) k_surf_vnormals(const float* __restrict__
 
 __global__ void k_surf_normals(const uint32_t* __restrict__ vslot, const float4* __restrict__ nslot,
                                float* __restrict__ nrm, uint32_t verts) {
+  chain_begin();
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= verts) return;
   const float4 n = nslot[vslot[tid]];
@@ -492,10 +499,11 @@ cudaError_t launch_surface_count(const Buffers& b, const DevParams& P, int cur, 
                                  cudaStream_t s) {
   const uint32_t cubes = static_cast<uint32_t>(g.nc[0]) * g.nc[1] * g.nc[2];
   const int64_t blocks = static_cast<int64_t>((g.nc[0] + 2) / 2) * ((g.nc[1] + 8) / 8) * ((g.nc[2] + 8) / 8);
-  k_surf_cells<<<blocks_for(b.n_cells, 256), 256, 0, s>>>(b.cell_start, b.scenes, any, b.n_cells);
-  k_surf_density<<<static_cast<unsigned>(blocks), 128, 0, s>>>(b.pos[cur], b.cell_start, b.scenes, any, g, field, P);
-  k_surf_count<<<surface_tiles(cubes), kCubeTile / 4, 0, s>>>(field, tab, g, iso, first, tile, cubes);
-  k_surf_tiles<<<1, 1024, 0, s>>>(tile, surface_tiles(cubes));
+  chain_launch(k_surf_cells, blocks_for(b.n_cells, 256), 256, 0, s, b.cell_start, b.scenes, any, b.n_cells);
+  chain_launch(k_surf_density, static_cast<unsigned>(blocks), 128, 0, s, b.pos[cur], b.cell_start, b.scenes, any, g,
+               field, P);
+  chain_launch(k_surf_count, surface_tiles(cubes), kCubeTile / 4, 0, s, field, tab, g, iso, first, tile, cubes);
+  chain_launch(k_surf_tiles, 1, 1024, 0, s, tile, surface_tiles(cubes));
   return cudaGetLastError();
 }
 
@@ -516,11 +524,11 @@ cudaError_t launch_surface_emit(const Buffers& b, const DevParams& P, int cur, c
   if (e == cudaSuccess) e = cudaMemsetAsync(hs.ucount, 0, sizeof(uint32_t), s);
   if (e != cudaSuccess) return e;
   const uint32_t verts = 3 * cap;
-  k_surf_vertices<<<blocks_for(verts, 128), 128, 0, s>>>(field, tab, g, iso, first, tile, cap, cubes, hs.keys,
-                                                         slots - 1, hs.vslot, hs.ulist, hs.ucount, xyz);
-  k_surf_vnormals<<<blocks_for(8ll * verts, 128), 128, 0, s>>>(field, g, iso, hs.keys, hs.ulist, hs.ucount, hs.nslot,
-                                                       b.pos[cur], b.cell_start, b.scenes, P);
-  k_surf_normals<<<blocks_for(verts, 256), 256, 0, s>>>(hs.vslot, hs.nslot, nrm, verts);
+  chain_launch(k_surf_vertices, blocks_for(verts, 128), 128, 0, s, field, tab, g, iso, first, tile, cap, cubes, hs.keys,
+               slots - 1, hs.vslot, hs.ulist, hs.ucount, xyz);
+  chain_launch(k_surf_vnormals, blocks_for(8ll * verts, 128), 128, 0, s, field, g, iso, hs.keys, hs.ulist, hs.ucount,
+               hs.nslot, b.pos[cur], b.cell_start, b.scenes, P);
+  chain_launch(k_surf_normals, blocks_for(verts, 256), 256, 0, s, hs.vslot, hs.nslot, nrm, verts);
   return cudaGetLastError();
 }
 
