@@ -30,6 +30,7 @@ constexpr int kMaxSums = 5;                            // accumulators of one wa
 constexpr int kRounds = 4;                             // pairs a lane evaluates between two exchanges
 constexpr uint32_t kDirectTiles = 16;                  // tiles up to which a block sums the counts before its own
 constexpr int kMaxPolls = 1 << 22;
+constexpr uint32_t kClusterBlocks = 16;
 
 struct SmallStep {
   const float4 *pos_a, *vel_a;
@@ -62,6 +63,27 @@ __device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, uns
   }
   __syncthreads();
   return passed;
+}
+
+// The same between the blocks of a cluster, in hardware. There every block keeps x* and the
+// displacements of the whole scene in its shared memory: a particle's team stores what it computes
+// into all blocks, and the neighbours' values are local loads.
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// dst: an address of this block's shared memory; v goes to it in blocks u, u + LANES, ... of the
+// cluster.
+template <int LANES>
+__device__ __forceinline__ void put_all(const void* dst, const float4& v, int u, unsigned blocks) {
+  const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
+  for (unsigned r = u; r < blocks; r += LANES) {
+    uint32_t at;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(a), "r"(r));
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+  }
 }
 
 // Exclusive scan over the block's threads; *total is the sum.
@@ -171,32 +193,39 @@ __device__ __forceinline__ float team_get(const float (&acc)[M], int a) {
   return __shfl_sync(0xffffffffu, acc[a / LANES], a & (LANES - 1), LANES);
 }
 
-template <int T, int LANES>
+template <int T, int LANES, bool CLUSTER>
 constexpr size_t small_smem() {
   if (LANES == 1) return sizeof(NbrWarp) * (T / 32);  // the lists take the tables' place
   const size_t lists = sizeof(uint16_t) * kOwnEntries * (T / LANES);
   const size_t bufs = sizeof(float2) * kMaxSums * (LANES * kRounds + 1) * (T / LANES);
   const size_t tables = sizeof(NbrWarp) * (T / LANES / 32);
-  return lists + (bufs > tables ? bufs : tables);
+  const size_t copies = CLUSTER ? 3 * sizeof(float4) * kClusterBlocks * (T / LANES) : 0;
+  return copies + lists + (bufs > tables ? bufs : tables);
 }
 
 // T threads a block. The first T / LANES of them also take one particle each in the stages before
 // the iterations: prediction, sort, neighbour build.
-template <int T, int LANES, bool N4>
+// CLUSTER: the grid is one thread block cluster and the barrier the cluster's own.
+template <int T, int LANES, bool N4, bool CLUSTER>
 __global__ void __launch_bounds__(T, 512 / T) k_step_small(const __grid_constant__ SmallStep A,
                                                             const __grid_constant__ DevParams P) {
   constexpr int kScanItems = static_cast<int>(kScanTile) / T;
   constexpr int PB = T / LANES;  // particles of a block
   extern __shared__ uint4 smem[];
-  uint16_t* lists = reinterpret_cast<uint16_t*>(smem);
+  constexpr int kCopy = CLUSTER ? static_cast<int>(kClusterBlocks) * PB : 0;  // particles of a cluster
+  float4* copies = reinterpret_cast<float4*>(smem);
+  uint16_t* lists = reinterpret_cast<uint16_t*>(copies + 3 * kCopy);
   char* work = reinterpret_cast<char*>(lists + (LANES == 1 ? 0 : kOwnEntries * PB));
   const unsigned full = 0xffffffffu;
   const unsigned G = gridDim.x;
   const int tid = static_cast<int>(threadIdx.x);
   const int n = A.n;
   unsigned target = 0;
-#define PBF_GRID_BARRIER() \
-  if (!grid_barrier(A.bar, target += G, A.err)) return
+#define PBF_GRID_BARRIER()                                       \
+  if constexpr (CLUSTER)                                         \
+    cluster_barrier();                                           \
+  else if (!grid_barrier(A.bar, target += G, A.err))             \
+    return
 
   // prediction (particles.cpp:175-183, 87-132) and cell counts
   const int i = static_cast<int>(blockIdx.x) * PB + tid;
@@ -297,10 +326,23 @@ __global__ void __launch_bounds__(T, 512 / T) k_step_small(const __grid_constant
   PBF_GRID_BARRIER();
 
   // neighbour lists of the block's slots
+  float4 *cur = A.xs0, *nxt = A.xs1, *disp = A.disp;
+  if constexpr (CLUSTER) {
+    cur = copies;
+    nxt = copies + kCopy;
+    disp = copies + 2 * kCopy;
+    for (int j = tid; j < n; j += T) {
+      cur[j] = A.xs0[j];
+      disp[j] = A.disp[j];
+    }
+  }
   if (front)
     nbr_build_warp<false>(reinterpret_cast<NbrWarp*>(work)[tid >> 5], i, A.xs0, A.pos_b, A.start, A.scenes, A.hdr,
                           A.words, A.err, P, A.one, n);
-  __syncthreads();
+  if constexpr (CLUSTER)
+    cluster_barrier();  // every block has its copies before another one stores into them
+  else
+    __syncthreads();
 
   // from here on a team of LANES lanes holds slot p
   const int team = tid / LANES, u = tid & (LANES - 1);
@@ -318,8 +360,8 @@ __global__ void __launch_bounds__(T, 512 / T) k_step_small(const __grid_constant
   if (act) {
     h = A.hdr[p];
     x4 = A.pos_b[p];
-    xi = A.xs0[p];
-    d = f3(A.disp[p]);
+    xi = cur[p];
+    d = f3(disp[p]);
   }
   const int total = nbr_total(h);
   const int most = __reduce_max_sync(full, total);
@@ -338,7 +380,6 @@ __global__ void __launch_bounds__(T, 512 / T) k_step_small(const __grid_constant
 
   // Jacobi iterations (particles.cpp:185-213). The first lambda pass needs no barrier: it reads
   // what the build read, and writes only its own x*.w.
-  float4 *cur = A.xs0, *nxt = A.xs1;
   auto load_x = [&](int e) -> float4 { return cur[slot(e)]; };
   for (int it = 0; it < A.iters; ++it) {
     {
@@ -362,8 +403,9 @@ __global__ void __launch_bounds__(T, 512 / T) k_step_small(const __grid_constant
       }
       float rho;
       xi.w = sum.lambda(P, &rho);
+      if (CLUSTER && act) put_all<LANES>(&cur[p], xi, u, G);
       if (lead) {
-        cur[p].w = xi.w;
+        if (!CLUSTER) cur[p].w = xi.w;
         if (it == 0 && A.rho_iter0) A.rho_iter0[p] = rho;
       }
     }
@@ -389,9 +431,13 @@ __global__ void __launch_bounds__(T, 512 / T) k_step_small(const __grid_constant
         collide<false, false>(x, d, sum.delta(P), false, sc, P);
         const float3 xn = displaced(x, d);
         xi = make_float4(xn.x, xn.y, xn.z, 0.f);
-        if (lead) {
+        const float4 d_out = make_float4(d.x, d.y, d.z, 0.f);
+        if (CLUSTER) {
+          put_all<LANES>(&nxt[p], xi, u, G);
+          if (it == A.iters - 1) put_all<LANES>(&disp[p], d_out, u, G);
+        } else if (lead) {
           nxt[p] = xi;
-          if (it == A.iters - 1) A.disp[p] = make_float4(d.x, d.y, d.z, 0.f);
+          if (it == A.iters - 1) disp[p] = d_out;
         }
       }
     }
@@ -405,11 +451,11 @@ __global__ void __launch_bounds__(T, 512 / T) k_step_small(const __grid_constant
   const float3 vi = d * A.inv_dt;
   auto load_xd = [&](int e) {
     const uint32_t j = slot(e);
-    return XD{cur[j], A.disp[j]};
+    return XD{cur[j], disp[j]};
   };
   XsphSum xs;
   if constexpr (LANES == 1) {
-    lane_walk<XD>(h, quad, [&](uint32_t j) { return XD{cur[j], A.disp[j]}; },
+    lane_walk<XD>(h, quad, [&](uint32_t j) { return XD{cur[j], disp[j]}; },
                   [&](const XD& q) { xs.add(xi, vi, q, A.inv_dt, P); });
   } else {
     float acc[(4 + LANES - 1) / LANES] = {};
@@ -434,8 +480,9 @@ __global__ void __launch_bounds__(T, 512 / T) k_step_small(const __grid_constant
     xs.w = make_float3(team_get<LANES>(acc, 0), team_get<LANES>(acc, 1), team_get<LANES>(acc, 2));
   }
   const float4 w = xs.omega(P);
+  if (CLUSTER && act) put_all<LANES>(&cur[p], make_float4(xi.x, xi.y, xi.z, w.w), u, G);
   if (lead) {
-    cur[p].w = w.w;
+    if (!CLUSTER) cur[p].w = w.w;
     A.rho[p] = xs.rho(P);
   }
   PBF_GRID_BARRIER();
@@ -465,23 +512,47 @@ __global__ void __launch_bounds__(T, 512 / T) k_step_small(const __grid_constant
   }
 #undef PBF_GRID_BARRIER
   // every block is past the last barrier when it counts itself out; the last one clears the count
-  if (tid == 0 && atomicInc(A.bar + 1, G - 1) == G - 1) *A.bar = 0u;
+  if (!CLUSTER && tid == 0 && atomicInc(A.bar + 1, G - 1) == G - 1) *A.bar = 0u;
 }
 
 using Kernel = void (*)(SmallStep, DevParams);
-template <int T, int LANES>
+template <int T, int LANES, bool CLUSTER>
 Kernel pick_kernel(bool n4) {
-  return n4 ? k_step_small<T, LANES, true> : k_step_small<T, LANES, false>;
+  return n4 ? k_step_small<T, LANES, true, CLUSTER> : k_step_small<T, LANES, false, CLUSTER>;
 }
 struct Form {
   Kernel kernel;
   uint32_t threads, per_block;  // threads and particles of a block
   size_t smem;
+  bool cluster;
 };
 Form pick(int form, bool n4) {
-  if (form == 1) return Form{pick_kernel<256, 8>(n4), 256, 32, small_smem<256, 8>()};
-  if (form == 2) return Form{pick_kernel<128, 1>(n4), 128, 128, small_smem<128, 1>()};
-  return Form{pick_kernel<256, 1>(n4), 256, 256, small_smem<256, 1>()};
+  switch (form) {
+    case 1: return Form{pick_kernel<512, 8, true>(n4), 512, 64, small_smem<512, 8, true>(), true};
+    case 2: return Form{pick_kernel<256, 8, false>(n4), 256, 32, small_smem<256, 8, false>(), false};
+    case 3: return Form{pick_kernel<128, 1, false>(n4), 128, 128, small_smem<128, 1, false>(), false};
+    default: return Form{pick_kernel<256, 1, false>(n4), 256, 256, small_smem<256, 1, false>(), false};
+  }
+}
+constexpr int kForms = 4;
+
+void set_config(const Form& f, uint32_t blocks, cudaStream_t s, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
+  *cfg = cudaLaunchConfig_t{};
+  cfg->gridDim = dim3(blocks);
+  cfg->blockDim = dim3(f.threads);
+  cfg->dynamicSmemBytes = f.smem;
+  cfg->stream = s;
+  *at = cudaLaunchAttribute{};
+  if (f.cluster) {
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = blocks;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  } else {
+    at->id = cudaLaunchAttributeCooperative;
+    at->val.cooperative = 1;
+  }
+  cfg->attrs = at;
+  cfg->numAttrs = 1;
 }
 
 }  // namespace
@@ -492,34 +563,45 @@ cudaError_t small_step_setup(int device, int* sms) {
   cudaError_t e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
   if (e != cudaSuccess || !coop) return e;
-  for (int form = 1; form <= 3; ++form)
+  for (int form = 1; form <= kForms; ++form)
     for (const bool n4 : {false, true}) {
       const Form f = pick(form, n4);
-      int per = 0;
       e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(f.smem));
-      if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f.kernel, static_cast<int>(f.threads), f.smem);
       if (e != cudaSuccess) return e;
-      if (per < (form == 1 ? 2 : 1)) return cudaSuccess;  // not used on this device
+      int fit = 0;
+      if (f.cluster) {
+        e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        set_config(f, kClusterBlocks, nullptr, &cfg, &at);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fit, f.kernel, &cfg);
+      } else {
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, f.kernel, static_cast<int>(f.threads), f.smem);
+        fit -= form == 2 ? 1 : 0;  // two blocks on an SM
+      }
+      if (e != cudaSuccess) return e;
+      if (fit < 1) return cudaSuccess;  // not used on this device
     }
   *sms = count;
   return cudaSuccess;
 }
 
-// Which form a scene takes; 0: the per-phase kernels. 8 lanes a particle while two blocks of 32
-// particles fit on every SM, then one lane a particle with one block on an SM. Steps (us, no
-// statistics) of 8 lanes / 1 lane / per-phase kernels: 512 particles 59 / 75 / 77, 4,096 65 / 85 /
-// 96, 8,000 73 / 87 / 101; 19k - / 89 / 105, 33k - / 89 / 109; with a second block on some SMs the
-// gain is gone (51k: 115 / 118). 4 lanes a particle: 8,000 77, 14k 93 (1 lane 89). Handles with
-// collider triangles or spheres keep the per-phase kernels: whether a move meets a triangle's edge
-// turns on the last bit, and the primitives' tests are not pinned to one rounding.
+// Which form a scene takes; 0: the per-phase kernels. One cluster of 16 blocks of 64 particles, 8
+// lanes each; the same over the grid while two blocks of 32 particles fit on every SM; then one lane
+// a particle with one block on an SM. Steps (us, no statistics) of 8 lanes over the grid /
+// 1 lane / per-phase kernels: 512 particles 59 / 75 / 77, 4,096 65 / 85 / 96, 8,000 73 / 87 / 101;
+// 19k - / 89 / 105, 33k - / 89 / 109; with a second block on some SMs the gain is gone (51k: 115 /
+// 118). 4 lanes a particle over the grid: 8,000 77, 14k 93 (1 lane 89). Handles with collider
+// triangles or spheres keep the per-phase kernels: whether a move meets a triangle's edge turns on
+// the last bit, and the primitives' tests are not pinned to one rounding.
 int small_step_form(const Buffers& b, const DevParams& P) {
   const size_t sms = static_cast<size_t>(b.small_sms);
   const size_t tiles = (static_cast<size_t>(b.n_cells) + kScanTile - 1) / kScanTile;
-  if (b.n == 0 || tiles > sms || P.n_mesh > 0 || P.n_sph > 0) return 0;
-  for (int form = 1; form <= 3; ++form) {
-    const size_t per_block = form == 1 ? 32 : form == 2 ? 128 : 256;
-    if ((b.n + per_block - 1) / per_block <= (form == 1 ? 2 * sms : sms)) return form;
+  if (b.n == 0 || P.n_mesh > 0 || P.n_sph > 0) return 0;
+  for (int form = 1; form <= kForms; ++form) {
+    const Form f = pick(form, true);
+    const size_t room = sms == 0 ? 0 : f.cluster ? kClusterBlocks : form == 2 ? 2 * sms : sms;
+    if ((b.n + f.per_block - 1) / f.per_block <= room && tiles <= room) return form;
   }
   return 0;
 }
@@ -559,16 +641,9 @@ cudaError_t launch_step_small(const Buffers& b, const DevParams& P, int form, in
   const uint32_t tiles = (a.m + kScanTile - 1) / kScanTile;
   const Form f = pick(form, P.scorr_n == 4);
   const uint32_t need = (static_cast<uint32_t>(b.n) + f.per_block - 1) / f.per_block;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(need > tiles ? need : tiles);
-  cfg.blockDim = dim3(f.threads);
-  cfg.dynamicSmemBytes = f.smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeCooperative;
-  at.val.cooperative = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  set_config(f, need > tiles ? need : tiles, s, &cfg, &at);
   return cudaLaunchKernelEx(&cfg, f.kernel, a, P);
 }
 

@@ -37,9 +37,9 @@ def _same(pos, vel, prm, **kw):
         np.testing.assert_array_equal(a, b)
 
 
-# 8 lanes a particle up to 2 x 152 blocks of 32, one lane up to 152 blocks of 128 and of 256, above
-# them the per-phase kernels
-@pytest.mark.parametrize("n", [1, 31, 33, 500, 9727, 9729, 19455, 19457, 38911, 38913])
+# a cluster up to 1,024 particles, 8 lanes a particle up to 2 x 152 blocks of 32, one lane up to 152
+# blocks of 128 and of 256, above them the per-phase kernels
+@pytest.mark.parametrize("n", [1, 31, 33, 64, 65, 500, 1024, 1025, 9727, 9729, 19455, 19457, 38911, 38913])
 def test_same_bits_at_the_ends_of_the_forms(n):
     pos, vel, h = _state(n, seed=n)
     _same(pos, vel, scenes.physical_params(h, h / 2, flags=PBF_FLAG_STATS, max_neighbors=256))
