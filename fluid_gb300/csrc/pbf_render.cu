@@ -527,12 +527,15 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want) {
 // Of hits at the same distance the last met still wins: the leaves keep their order, and
 // one that an earlier test would have culled lies behind the nearest hit. Steps a turn at
 // 1280x720, 32 samples, 1 M particles (tracing, ms; 14.3 with tests at once, the rays
-// begun as under k_wf_trace): 12.9 with 4, 12.6 with 6, 13.0 with 8, 14.3 with 12. What
-// bounds it now is the L1 data pipe (78% of its cycles: 16-byte gathers of nodes), at 41%
-// of the warps (60 and 72 registers; fewer spill: 14.3 ms at 10 blocks an SM). Phase 0 walks the
-// scene's tree (when the scene has one), phase 1 the surface's; phase 2 is done.
+// begun as under k_wf_trace): 12.9 with 4, 12.6 with 6, 13.0 with 8, 14.3 with 12. The L1
+// data pipe then took 78% of the cycles (16-byte gathers of nodes, and the lanes' stacks in
+// local memory, a line for every depth in the warp), so the first kNearStack levels of the
+// stack are in shared memory, a bank a lane: 12.55 -> 11.7 ms (8 to 12 levels; 11.8 with 16).
+// More blocks an SM than its 62 and 72 registers allow: 12.1 ms with 8, 12.7 with 9. Phase
+// 0 walks the scene's tree (when the scene has one), phase 1 the surface's; 2 is done.
 constexpr int kWalkThreads = 128;
 constexpr int kWalkSteps = 6;
+constexpr int kNearStack = 8;
 constexpr uint32_t kNoNode = 0xffffffffu;
 struct Walk {
   uint32_t node;  // kNoNode: the tree of this phase is walked
@@ -541,7 +544,7 @@ struct Walk {
   int best;
   int leaves;
   float tmax, bu, bv;
-  uint32_t stack[kBvhStack];
+  uint32_t deep[kBvhStack - kNearStack];
 };
 
 // Enters the first tree from s.phase on with more than one triangle (a tree of one is
@@ -591,7 +594,8 @@ __device__ __forceinline__ void walk_begin(const Scene& sc, const Ray& r, Walk& 
 // One node of the current tree: both children's boxes; leaves are collected in
 // queue[.][thread], the nearer hit child comes next and the farther one is pushed.
 __device__ __forceinline__ void walk_node(const Scene& sc, const Ray& r, Walk& s,
-                                          uint32_t (&queue)[2 * kWalkSteps][kWalkThreads], unsigned* err) {
+                                          uint32_t (&queue)[2 * kWalkSteps][kWalkThreads],
+                                          uint32_t (&stack)[kNearStack][kWalkThreads], unsigned* err) {
   const bool scene = s.phase == 0;
   const BvhNode* __restrict__ nodes = scene ? sc.scene_nodes : sc.surf_nodes;
   const BvhNode nd = nodes[s.node];
@@ -609,8 +613,11 @@ __device__ __forceinline__ void walk_node(const Scene& sc, const Ray& r, Walk& s
   }
   if (hl && hr) {
     const bool lfirst = tl <= tr;
-    if (s.sp < kBvhStack) {
-      s.stack[s.sp++] = lfirst ? cr : cl;
+    const uint32_t later = lfirst ? cr : cl;
+    if (s.sp < kNearStack) {
+      stack[s.sp++][threadIdx.x] = later;
+    } else if (s.sp < kBvhStack) {
+      s.deep[s.sp++ - kNearStack] = later;
     } else {
       atomicOr(err, 1u);
     }
@@ -620,7 +627,8 @@ __device__ __forceinline__ void walk_node(const Scene& sc, const Ray& r, Walk& s
   } else if (hr) {
     s.node = cr;
   } else if (s.sp > 0) {
-    s.node = s.stack[--s.sp];
+    --s.sp;
+    s.node = s.sp < kNearStack ? stack[s.sp][threadIdx.x] : s.deep[s.sp - kNearStack];
   } else {
     s.node = kNoNode;
   }
@@ -684,6 +692,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_wf_trace(Scene sc, WfArgs w, c
   const unsigned full = 0xffffffffu, lane = threadIdx.x & 31u;
   const uint32_t total = *count;
   __shared__ uint32_t queue_leaves[2 * kWalkSteps][kWalkThreads];
+  __shared__ uint32_t near_stack[kNearStack][kWalkThreads];
   __shared__ WaitingRays waiting[kWalkThreads / 32];
   WaitingRays& wait = waiting[threadIdx.x >> 5];
   int head = 0, waits = 0;
@@ -756,7 +765,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_wf_trace(Scene sc, WfArgs w, c
     }
     if (need == full) break;
     for (int k = 0; k < kWalkSteps; ++k)
-      if (s.phase < 2 && s.node != kNoNode) walk_node(sc, r, s, queue_leaves, err);
+      if (s.phase < 2 && s.node != kNoNode) walk_node(sc, r, s, queue_leaves, near_stack, err);
     walk_leaves<ANY>(sc, r, s, queue_leaves);
     if (s.phase < 2 && s.node == kNoNode) {
       ++s.phase;
