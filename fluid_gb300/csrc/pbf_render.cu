@@ -878,7 +878,9 @@ __global__ void __launch_bounds__(128) k_wf_shade(Scene sc, WfArgs w, RArgs a, i
             const V3 c = mulv(beta, mulv(Ls, fval) * (fabsf(cz_in) / pdf));
             con = make_float4(c.x / ns, c.y / ns, c.z / ns, 0.f);
             dir4 = make_float4(wi.x, wi.y, wi.z, dist);
-            want = true;
+            // a sample that adds nothing (the back of an area light) needs no visibility: 11.76 ->
+            // 11.42 ms of tracing at 1280x720, 32 samples; NaN is traced as before
+            want = !(con.x == 0.f && con.y == 0.f && con.z == 0.f);
           }
         }
         if (hit) {
