@@ -267,7 +267,7 @@ __global__ void k_tree(const uint32_t* __restrict__ keys, int n, BvhNode* __rest
   const uint32_t right = (max(i, j) == gamma + 1) ? (kLeafBit | static_cast<uint32_t>(gamma + 1))
                                                   : static_cast<uint32_t>(gamma + 1);
   nodes[i].lo_l.w = __uint_as_float(left);
-  nodes[i].lo_r.w = __uint_as_float(right);
+  nodes[i].hi_l.w = __uint_as_float(right);
   parent[(left & kLeafBit) ? (n - 1 + (left & ~kLeafBit)) : left] = static_cast<uint32_t>(i);
   parent[(right & kLeafBit) ? (n - 1 + (right & ~kLeafBit)) : right] = static_cast<uint32_t>(i);
   if (i == 0) parent[0] = 0xffffffffu;
@@ -295,15 +295,15 @@ __global__ void k_refit(const RTri* __restrict__ tri, const uint32_t* __restrict
     __threadfence();
     if (atomicAdd(&flags[p], 1u) == 0u) return;  // the sibling finishes this node
     __threadfence();
-    const uint32_t cl = __float_as_uint(__ldcg(&nodes[p].lo_l.w)), cr = __float_as_uint(__ldcg(&nodes[p].lo_r.w));
+    const uint32_t cl = __float_as_uint(__ldcg(&nodes[p].lo_l.w)), cr = __float_as_uint(__ldcg(&nodes[p].hi_l.w));
     const uint32_t bl = (cl & kLeafBit) ? static_cast<uint32_t>(n - 1) + (cl & ~kLeafBit) : cl;
     const uint32_t br = (cr & kLeafBit) ? static_cast<uint32_t>(n - 1) + (cr & ~kLeafBit) : cr;
     const float4 ll = __ldcg(&box_lo[bl]), lh = __ldcg(&box_hi[bl]);
     const float4 rl = __ldcg(&box_lo[br]), rh = __ldcg(&box_hi[br]);
     nodes[p].lo_l = make_float4(ll.x, ll.y, ll.z, __uint_as_float(cl));
-    nodes[p].hi_l = lh;
-    nodes[p].lo_r = make_float4(rl.x, rl.y, rl.z, __uint_as_float(cr));
-    nodes[p].hi_r = rh;
+    nodes[p].hi_l = make_float4(lh.x, lh.y, lh.z, __uint_as_float(cr));
+    nodes[p].lo_r = make_float4(rl.x, rl.y, rl.z, rh.x);
+    nodes[p].hi_r_yz = make_float2(rh.y, rh.z);
     box_lo[p] = make_float4(fminf(ll.x, rl.x), fminf(ll.y, rl.y), fminf(ll.z, rl.z), 0.f);
     box_hi[p] = make_float4(fmaxf(lh.x, rh.x), fmaxf(lh.y, rh.y), fmaxf(lh.z, rh.z), 0.f);
     p = parent[p];
@@ -598,11 +598,13 @@ __device__ __forceinline__ void walk_node(const Scene& sc, const Ray& r, Walk& s
                                           uint32_t (&stack)[kNearStack][kWalkThreads], unsigned* err) {
   const bool scene = s.phase == 0;
   const BvhNode* __restrict__ nodes = scene ? sc.scene_nodes : sc.surf_nodes;
-  const BvhNode nd = nodes[s.node];
+  const BvhNode& nd = nodes[s.node];
+  const float4 lo_l = __ldg(&nd.lo_l), hi_l = __ldg(&nd.hi_l), lo_r = __ldg(&nd.lo_r);
+  const float2 yz = __ldg(&nd.hi_r_yz);
   float tl, tr;
-  bool hl = box_test(nd.lo_l, nd.hi_l, r, s.tmax, &tl);
-  bool hr = box_test(nd.lo_r, nd.hi_r, r, s.tmax, &tr);
-  const uint32_t cl = __float_as_uint(nd.lo_l.w), cr = __float_as_uint(nd.lo_r.w);
+  bool hl = box_test(lo_l, hi_l, r, s.tmax, &tl);
+  bool hr = box_test(lo_r, make_float4(lo_r.w, yz.x, yz.y, 0.f), r, s.tmax, &tr);
+  const uint32_t cl = __float_as_uint(lo_l.w), cr = __float_as_uint(hi_l.w);
   if (hl && (cl & kLeafBit)) {
     queue[s.leaves++][threadIdx.x] = cl & ~kLeafBit;
     hl = false;
@@ -730,7 +732,8 @@ __global__ void __launch_bounds__(kWalkThreads) k_wf_trace(Scene sc, WfArgs w, c
             const BvhNode nd = sc.surf_nodes[0];
             float tl, tr;
             const bool hl = box_test(nd.lo_l, nd.hi_l, b, ws.tmax, &tl);
-            walks = hl || box_test(nd.lo_r, nd.hi_r, b, ws.tmax, &tr);
+            const float4 hi_r = make_float4(nd.lo_r.w, nd.hi_r_yz.x, nd.hi_r_yz.y, 0.f);
+            walks = hl || box_test(nd.lo_r, hi_r, b, ws.tmax, &tr);
           }
           if (!walks) trace_result<ANY>(w, q, ws);
         }
