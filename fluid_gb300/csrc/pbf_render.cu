@@ -526,7 +526,7 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want) {
 // 130 instead of 212 million instructions (first bounce of 640x360 at 8 samples).
 // Of hits at the same distance the last met still wins: the leaves keep their order, and
 // one that an earlier test would have culled lies behind the nearest hit. Steps a turn at
-// 1280x720, 32 samples, 1 M particles (tracing, ms; 14.3 with tests at once, the rays
+// 1280x720, 16 samples, 1 M particles (tracing, ms; 14.3 with tests at once, the rays
 // begun as under k_wf_trace): 12.9 with 4, 12.6 with 6, 13.0 with 8, 14.3 with 12. The L1
 // data pipe then took 78% of the cycles (16-byte gathers of nodes, and the lanes' stacks in
 // local memory, a line for every depth in the warp), so the first kNearStack levels of the
@@ -882,7 +882,7 @@ __global__ void __launch_bounds__(128) k_wf_shade(Scene sc, WfArgs w, RArgs a, i
             con = make_float4(c.x / ns, c.y / ns, c.z / ns, 0.f);
             dir4 = make_float4(wi.x, wi.y, wi.z, dist);
             // a sample that adds nothing (the back of an area light) needs no visibility: 11.76 ->
-            // 11.42 ms of tracing at 1280x720, 32 samples; NaN is traced as before
+            // 11.42 ms of tracing at 1280x720, 16 samples; NaN is traced as before
             want = !(con.x == 0.f && con.y == 0.f && con.z == 0.f);
           }
         }

@@ -23,7 +23,7 @@ struct RNrm {
 // Internal node of the BVH: the boxes of both children; lo_l.w / hi_l.w hold the left / right
 // child's index (int bits), leaves (triangles) tagged with kLeafBit; lo_r.w is the right box's
 // upper x. A walk so reads 56 bytes a node instead of 64 (11.38 -> 11.22 ms of tracing at
-// 1280x720, 32 samples, bound by the L1 data pipe).
+// 1280x720, 16 samples, bound by the L1 data pipe).
 struct BvhNode {
   float4 lo_l, hi_l, lo_r;
   float2 hi_r_yz, unused;

@@ -190,7 +190,8 @@ PBF_API pbf_status pbf_get_predicted(pbf_handle* h, float* xyz);
 /*
  * Per-phase CUDA-event timing (the reference times nothing on this path; it
  * prints progress, particles.cpp:251-295). While enabled, steps run without
- * graph replay and record an event after each phase on the handle's stream.
+ * graph replay and record an event after each phase on the handle's stream; a
+ * small scene, whose step is otherwise one launch, then runs a launch per phase.
  * pbf_get_phase_times waits and returns, per phase, the accumulated device
  * milliseconds and the number of kernel launches since the last reset.
  */
@@ -204,7 +205,8 @@ PBF_API const char* pbf_phase_name(int phase);
 /*
  * Launch shapes (threads per block) of the kernel families of a step, and the
  * forms of the neighbour kernels. No field changes any result bit: the forms
- * visit every particle's neighbours in the same order.
+ * visit every particle's neighbours in the same order. The step of a small scene
+ * (one launch) has its own shapes and takes none of these.
  */
 typedef struct pbf_tuning {
   int32_t block_predict;  /* prediction, cell count */
