@@ -709,6 +709,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_wf_trace(Scene sc, WfArgs w, c
     unsigned need = __ballot_sync(full, item == kNoItem);
     while (need && (head < waits || !drained)) {
       if (head == waits) {
+        __syncwarp(full);  // the rays handed out before are read
         uint32_t first = 0;
         if (lane == 0) first = atomicAdd(fetch, 32u);
         first = __shfl_sync(full, first, 0);
