@@ -175,7 +175,7 @@ void Handle::free_all() {
   void* ptrs[] = {b.pos[0], b.pos[1], b.disp[0], b.disp[1], b.xs[0], b.xs[1], b.vel[0], b.vel[1],
                   b.omega, b.pred, b.xkey, b.rho, b.rho_iter0, b.id[0], b.id[1], b.key, b.rank,
                   b.perm, b.perm_atomic, b.nbr_hdr, b.nbr_w, b.cell_count, b.cell_start, b.scan_tmp, b.big_cells, b.big_count, b.scenes, b.stats_part,
-                  b.stats, b.err, b.grid_bar, b.io, b.io2, scratch, snap_pos, snap_vel, snap_id};
+                  b.stats, b.err, b.io, b.io2, scratch, snap_pos, snap_vel, snap_id};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   b = Buffers();
@@ -223,7 +223,7 @@ pbf_status Handle::alloc_all() {
       {(void**)&b.big_count, sizeof(uint32_t)},
       {(void**)&b.scenes, sizeof(SceneDesc) * b.n_scenes}, {(void**)&b.stats, sizeof(DevStats)},
       {(void**)&b.stats_part, sizeof(DevStats) * kStatsBlocks},
-      {(void**)&b.err, sizeof(unsigned)}, {(void**)&b.grid_bar, 3 * sizeof(unsigned)}, {(void**)&b.io, 3 * sizeof(float) * n},
+      {(void**)&b.err, 4 * sizeof(unsigned)}, {(void**)&b.io, 3 * sizeof(float) * n},
       {(void**)&b.io2, 3 * sizeof(float) * n},
   };
   for (auto& a : list) {
@@ -237,10 +237,10 @@ pbf_status Handle::alloc_all() {
   pbf_status st = cuda(cudaMemsetAsync(b.scan_tmp, 0, sizeof(uint32_t) * ((b.n_cells + 1023) / 1024 + 1), stream),
                        "cudaMemsetAsync");  // the scan's ticket word (after the tile sums) starts at zero
   if (st == PBF_OK) st = cuda(cudaMemsetAsync(b.cell_count, 0, sizeof(uint32_t) * b.n_cells, stream), "cudaMemsetAsync");
-  if (st == PBF_OK) st = cuda(cudaMemsetAsync(b.grid_bar, 0, 3 * sizeof(unsigned), stream), "cudaMemsetAsync");
-  if (st == PBF_OK) st = cuda(small_step_setup(device, &b.small_sms), "occupancy");
+  b.grid_bar = b.err + 1;
+  if (st == PBF_OK) st = cuda(small_step_setup(device, dp, &b), "occupancy");
   if (st != PBF_OK) return st;
-  return cuda(cudaMemsetAsync(b.err, 0, sizeof(unsigned), stream), "cudaMemsetAsync");
+  return cuda(cudaMemsetAsync(b.err, 0, 4 * sizeof(unsigned), stream), "cudaMemsetAsync");
 }
 
 void Handle::free_tape() {

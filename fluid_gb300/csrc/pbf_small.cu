@@ -555,37 +555,6 @@ void set_config(const Form& f, uint32_t blocks, cudaStream_t s, cudaLaunchConfig
   cfg->numAttrs = 1;
 }
 
-}  // namespace
-
-cudaError_t small_step_setup(int device, int* sms) {
-  *sms = 0;
-  int count = 0, coop = 0;
-  cudaError_t e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
-  if (e != cudaSuccess || !coop) return e;
-  for (int form = 1; form <= kForms; ++form)
-    for (const bool n4 : {false, true}) {
-      const Form f = pick(form, n4);
-      e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(f.smem));
-      if (e != cudaSuccess) return e;
-      int fit = 0;
-      if (f.cluster) {
-        e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        cudaLaunchConfig_t cfg;
-        cudaLaunchAttribute at;
-        set_config(f, kClusterBlocks, nullptr, &cfg, &at);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fit, f.kernel, &cfg);
-      } else {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, f.kernel, static_cast<int>(f.threads), f.smem);
-        fit -= form == 2 ? 1 : 0;  // two blocks on an SM
-      }
-      if (e != cudaSuccess) return e;
-      if (fit < 1) return cudaSuccess;  // not used on this device
-    }
-  *sms = count;
-  return cudaSuccess;
-}
-
 // Which form a scene takes; 0: the per-phase kernels. One cluster of 16 blocks of 64 particles, 8
 // lanes each; the same over the grid while two blocks of 32 particles fit on every SM; then one lane
 // a particle with one block on an SM. Steps (us, no statistics) of 8 lanes over the grid /
@@ -594,16 +563,48 @@ cudaError_t small_step_setup(int device, int* sms) {
 // 118). 4 lanes a particle over the grid: 8,000 77, 14k 93 (1 lane 89). Handles with collider
 // triangles or spheres keep the per-phase kernels: whether a move meets a triangle's edge turns on
 // the last bit, and the primitives' tests are not pinned to one rounding.
-int small_step_form(const Buffers& b, const DevParams& P) {
-  const size_t sms = static_cast<size_t>(b.small_sms);
-  const size_t tiles = (static_cast<size_t>(b.n_cells) + kScanTile - 1) / kScanTile;
-  if (b.n == 0 || P.n_mesh > 0 || P.n_sph > 0) return 0;
-  for (int form = 1; form <= kForms; ++form) {
+int form_for(size_t n, size_t n_cells, size_t sms) {
+  const size_t tiles = (n_cells + kScanTile - 1) / kScanTile;
+  for (int form = 1; n > 0 && sms > 0 && form <= kForms; ++form) {
     const Form f = pick(form, true);
-    const size_t room = sms == 0 ? 0 : f.cluster ? kClusterBlocks : form == 2 ? 2 * sms : sms;
-    if ((b.n + f.per_block - 1) / f.per_block <= room && tiles <= room) return form;
+    const size_t room = f.cluster ? kClusterBlocks : form == 2 ? 2 * sms : sms;
+    if ((n + f.per_block - 1) / f.per_block <= room && tiles <= room) return form;
   }
   return 0;
+}
+
+}  // namespace
+
+// Only the kernel that this handle would launch is looked at: each look costs a handle's creation
+// tens of microseconds, and the first one loads the kernel.
+cudaError_t small_step_setup(int device, const DevParams& P, Buffers* b) {
+  b->small_sms = 0;
+  int count = 0, coop = 0, fit = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
+  if (e != cudaSuccess || !coop) return e;
+  const int form = form_for(b->n, b->n_cells, static_cast<size_t>(count));
+  if (form == 0) return cudaSuccess;
+  const Form f = pick(form, P.scorr_n == 4);
+  e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(f.smem));
+  if (e != cudaSuccess) return e;
+  if (f.cluster) {
+    e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at;
+    set_config(f, kClusterBlocks, nullptr, &cfg, &at);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fit, f.kernel, &cfg);
+  } else {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, f.kernel, static_cast<int>(f.threads), f.smem);
+    fit -= form == 2 ? 1 : 0;  // two blocks on an SM
+  }
+  if (e == cudaSuccess && fit >= 1) b->small_sms = count;
+  return e;
+}
+
+int small_step_form(const Buffers& b, const DevParams& P) {
+  if (P.n_mesh > 0 || P.n_sph > 0) return 0;
+  return form_for(b.n, b.n_cells, static_cast<size_t>(b.small_sms));
 }
 
 cudaError_t launch_step_small(const Buffers& b, const DevParams& P, int form, int cur, float dt, int iters,
