@@ -239,6 +239,12 @@ pbf_status Handle::alloc_all() {
   if (st == PBF_OK) st = cuda(cudaMemsetAsync(b.cell_count, 0, sizeof(uint32_t) * b.n_cells, stream), "cudaMemsetAsync");
   b.grid_bar = b.err + 1;
   if (st == PBF_OK) st = cuda(small_step_setup(device, dp, &b), "occupancy");
+  if (st == PBF_OK && small_step_waits(small_step_form(b, dp))) {
+    // the second buffers hold valid indexes before their first step: what follows a step that gave
+    // up (usable) reads them
+    st = cuda(cudaMemsetAsync(b.pos[1], 0, sizeof(float4) * n, stream), "cudaMemsetAsync");
+    if (st == PBF_OK) st = cuda(cudaMemsetAsync(b.id[1], 0, sizeof(uint32_t) * n, stream), "cudaMemsetAsync");
+  }
   if (st != PBF_OK) return st;
   return cuda(cudaMemsetAsync(b.err, 0, 4 * sizeof(unsigned), stream), "cudaMemsetAsync");
 }
@@ -305,7 +311,9 @@ pbf_status Handle::sync_and_check() {
   if (st != PBF_OK) return st;
   st = cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
   if (st != PBF_OK) return st;
-  if (host_err_word & PBF_ERRBIT_TIMEOUT) return fail(PBF_ERR_TIMEOUT, "a wait of the step's grid barrier gave up");
+  st = usable();
+  if (st != PBF_OK) return st;
+  counts_open = false;
   if (host_err_word & PBF_ERRBIT_NONFINITE) return fail(PBF_ERR_NONFINITE, "a position or velocity became non-finite");
   if (host_err_word & PBF_ERRBIT_NEIGHBOR_CAPACITY)
     return fail(PBF_ERR_CAPACITY, "a particle had more neighbours than max_neighbors");
@@ -314,6 +322,31 @@ pbf_status Handle::sync_and_check() {
                 "more than 4096 particles in one 3-cell row, or a neighbour more than 16383 slots past its "
                 "z-slab's first candidate");
   return PBF_OK;
+}
+
+// After a wait inside a step has given up, the state is neither the old nor the new one, and stays
+// so: calls that read it are refused. Work enqueued before the host knows stays in bounds: later
+// whole-step launches return at once, the cell counts are cleared (close_counts), and every index
+// in the buffers is a valid one.
+pbf_status Handle::usable() {
+  if (!(host_err_word & PBF_ERRBIT_TIMEOUT)) return PBF_OK;
+  return fail(PBF_ERR_TIMEOUT, "a wait of the step's grid barrier gave up: the handle stays failed");
+}
+
+pbf_status Handle::close_counts() {
+  if (!counts_open) return PBF_OK;
+  counts_open = false;
+  return cuda(cudaMemsetAsync(b.cell_count, 0, sizeof(uint32_t) * b.n_cells, stream), "cudaMemsetAsync");
+}
+
+pbf_status Handle::resort() {
+  pbf_status st = usable();
+  if (st == PBF_OK) st = close_counts();
+  if (st == PBF_OK) st = cuda(launch_resort(b, dp, tune, cur, stream), "resort");
+  if (st != PBF_OK) return st;
+  cur ^= 1;
+  nbr_valid = false;
+  return st;
 }
 
 PhaseMarks Handle::next_marks() {
@@ -384,6 +417,12 @@ static pbf_status capture_step(Handle* h, float dt, bool keep_pred, PhaseMarks* 
 }
 
 pbf_status Handle::enqueue_steps(float dt, int nsteps) {
+  pbf_status ok = usable();
+  if (ok != PBF_OK) return ok;
+  const int form = profiling ? 0 : small_step_form(b, dp);
+  if (form == 0 && nsteps > 0) ok = close_counts();
+  if (ok != PBF_OK) return ok;
+  if (small_step_waits(form) && nsteps > 0) counts_open = true;
   const bool use_graph = (params.flags & PBF_FLAG_GRAPH) != 0;
   const bool keep_pred = b.pred != nullptr;
   const int it = params.iters;
@@ -661,9 +700,11 @@ pbf_status pbf_adjoint_step_device(pbf_handle* hh, double dt, const float* xyz, 
     return h->fail(PBF_ERR_INVALID, "the adjoint step supports the box collider only");
   if (h->b.n && (!gx_in || !gv_in)) return h->fail(PBF_ERR_INVALID, "gx_in / gv_in is NULL");
   pbf::DeviceGuard g(h->device);
-  pbf_status st = h->ensure_tape();
+  pbf_status st = h->usable();
+  if (st == PBF_OK) st = h->ensure_tape();
   if (st != PBF_OK) return st;
   st = h->join_from(static_cast<cudaStream_t>(stream));
+  if (st == PBF_OK) st = h->close_counts();
   if (st != PBF_OK) return st;
   if (xyz) {
     st = h->cuda(pbf::launch_upload(h->b, h->cur, xyz, vel, nullptr, h->stream), "upload");
@@ -693,7 +734,9 @@ static pbf_status download(Handle* h, float* xyz, float* vel, float* rho) {
   const size_t n = h->b.n;
   if (n == 0 || (!xyz && !vel && !rho)) return PBF_OK;
   float* tmp = reinterpret_cast<float*>(h->b.disp[0]);  // scratch between steps
-  pbf_status st = h->cuda(pbf::launch_download(h->b, h->cur, xyz ? h->b.io : nullptr, vel ? h->b.io2 : nullptr,
+  pbf_status st = h->usable();
+  if (st != PBF_OK) return st;
+  st = h->cuda(pbf::launch_download(h->b, h->cur, xyz ? h->b.io : nullptr, vel ? h->b.io2 : nullptr,
                                                rho ? tmp : nullptr, h->stream),
                           "download");
   if (st == PBF_OK && xyz)
@@ -760,7 +803,8 @@ pbf_status pbf_get_state_device(pbf_handle* hh, float* xyz, float* vel, float* r
   if (!hh) return PBF_ERR_INVALID;
   Handle* h = reinterpret_cast<Handle*>(hh);
   pbf::DeviceGuard g(h->device);
-  pbf_status st = h->join_from(static_cast<cudaStream_t>(stream));
+  pbf_status st = h->usable();
+  if (st == PBF_OK) st = h->join_from(static_cast<cudaStream_t>(stream));
   if (st == PBF_OK)
     st = h->cuda(pbf::launch_download(h->b, h->cur, xyz, vel, rho, h->stream), "download");
   if (st == PBF_OK) st = h->join_to(static_cast<cudaStream_t>(stream));
@@ -772,10 +816,8 @@ pbf_status pbf_estimate_densities(pbf_handle* hh, float* rho) {
   Handle* h = reinterpret_cast<Handle*>(hh);
   pbf::DeviceGuard g(h->device);
   if (h->b.n == 0) return PBF_OK;
-  pbf_status st = h->cuda(pbf::launch_resort(h->b, h->dp, h->tune, h->cur, h->stream), "resort");
+  pbf_status st = h->resort();
   if (st != PBF_OK) return st;
-  h->cur ^= 1;
-  h->nbr_valid = false;
   h->drop_graphs();
   st = h->cuda(pbf::launch_density_self(h->b, h->dp, h->tune, h->cur, h->b.rho, h->stream), "density");
   if (st != PBF_OK) return st;
@@ -1006,10 +1048,8 @@ pbf_status Handle::surface_count(double isolevel, double step, const double* lo,
   if (cubes > 2.0e9) return fail(PBF_ERR_INVALID, "surface grid too large");
   *total = 0;
   if (b.n == 0) return PBF_OK;
-  pbf_status st = cuda(launch_resort(b, dp, tune, cur, stream), "resort");
+  pbf_status st = resort();
   if (st != PBF_OK) return st;
-  cur ^= 1;
-  nbr_valid = false;
   drop_graphs();
   if (!surf_table_dev) {
     st = cuda(cudaMalloc(&surf_table_dev, sizeof(SurfTable)), "cudaMalloc(table)");
@@ -1117,10 +1157,8 @@ pbf_status pbf_estimate_density_at(pbf_handle* hh, size_t m, const float* pts, f
   float* dpts = static_cast<float*>(h->scratch);
   float* dout = dpts + 3 * m;
   if (h->b.n) {
-    st = h->cuda(pbf::launch_resort(h->b, h->dp, h->tune, h->cur, h->stream), "resort");
+    st = h->resort();
     if (st != PBF_OK) return st;
-    h->cur ^= 1;
-    h->nbr_valid = false;
     h->drop_graphs();
   }
   st = h->cuda(cudaMemcpyAsync(dpts, pts, 3 * sizeof(float) * m, cudaMemcpyHostToDevice, h->stream), "H2D");
@@ -1151,6 +1189,7 @@ pbf_status pbf_get_stats(pbf_handle* hh, pbf_stats* out) {
   if (st == PBF_OK) st = h->cuda(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
   if (st != PBF_OK) return st;
   out->error_flags = errw;
+  h->host_err_word |= errw & PBF_ERRBIT_TIMEOUT;
   if (!h->dp.stats || h->steps == 0 || h->b.n == 0) return PBF_OK;
   const double n = static_cast<double>(h->b.n);
   out->mean_density_iter0 = ds.rho_iter0_sum / n;
@@ -1176,7 +1215,11 @@ pbf_status pbf_get_neighbors(pbf_handle* hh, uint32_t* counts, uint32_t* ids, si
     if (total) *total = 0;
     return PBF_OK;
   }
-  pbf_status st = h->ensure_scratch(sizeof(uint32_t) * (2 * n + 1));
+  pbf_status st = PBF_OK;
+  if (h->counts_open) st = h->sync_and_check();  // a step that gave up leaves no lists to read
+  if (st == PBF_OK || st == PBF_ERR_NONFINITE || st == PBF_ERR_CAPACITY) st = h->usable();
+  if (st != PBF_OK) return st;
+  st = h->ensure_scratch(sizeof(uint32_t) * (2 * n + 1));
   if (st != PBF_OK) return st;
   uint32_t* dcounts = static_cast<uint32_t*>(h->scratch);
   st = h->cuda(pbf::launch_neighbor_counts(h->b, h->cur, dcounts, h->stream), "counts");
@@ -1237,10 +1280,8 @@ pbf_status pbf_sort(pbf_handle* hh) {
   Handle* h = reinterpret_cast<Handle*>(hh);
   pbf::DeviceGuard g(h->device);
   if (h->b.n == 0) return PBF_OK;
-  pbf_status st = h->cuda(pbf::launch_resort(h->b, h->dp, h->tune, h->cur, h->stream), "resort");
+  pbf_status st = h->resort();
   if (st != PBF_OK) return st;
-  h->cur ^= 1;
-  h->nbr_valid = false;
   return h->cuda(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
 }
 
@@ -1316,6 +1357,14 @@ pbf_status pbf_set_tuning(pbf_handle* hh, const pbf_tuning* t) {
   h->tune.gather_depth = t->gather_depth;
   h->tune.list_stream = t->list_stream;
   h->drop_graphs();
+  return PBF_OK;
+}
+
+pbf_status pbf_set_wait_limit(pbf_handle* hh, uint32_t reads) {
+  if (!hh) return PBF_ERR_INVALID;
+  Handle* h = reinterpret_cast<Handle*>(hh);
+  h->b.wait_reads = reads;
+  h->drop_graphs();  // a captured step holds the limit
   return PBF_OK;
 }
 

@@ -36,6 +36,8 @@ struct Handle {
   bool nbr_valid = false;    // neighbour lists / x* copy describe the current order
   std::string err;
   unsigned host_err_word = 0;
+  bool counts_open = false;  // a whole-step launch that may have given up has not been checked: its cell counts
+                             // may not be zero
   cudaGraphExec_t graph[2] = {nullptr, nullptr};  // one step starting from buffers 0 / 1
   float graph_dt = -1.f;
   void* scratch = nullptr;   // grow-only scratch for introspection and queries
@@ -84,6 +86,9 @@ struct Handle {
   pbf_status surface_emit(const SurfGrid& g, double isolevel, float* xyz, float* nrm, uint32_t cap);
   pbf_status enqueue_steps(float dt, int nsteps);
   pbf_status sync_and_check();
+  pbf_status usable();        // PBF_ERR_TIMEOUT once a wait is known to have given up
+  pbf_status close_counts();  // before a per-phase kernel counts into the cells
+  pbf_status resort();        // the current state into cell order
   void drop_graphs();
   PhaseMarks next_marks();
   pbf_status collect_phase_times();

@@ -117,6 +117,7 @@ struct Buffers {
   unsigned int* grid_bar = nullptr;  // counters, zero between launches: the whole-step kernel's barrier and the
                                      // blocks that left it, the statistics pass's ticket
   int small_sms = 0;                 // SMs for the whole-step kernel (0: not used)
+  unsigned wait_reads = 0;           // reads after which a wait inside a step gives up (0: 4 million)
   float* io = nullptr;             // (n, 3) staging for host/device packed transfers
   float* io2 = nullptr;
 };
@@ -231,6 +232,7 @@ cudaError_t launch_adjoint(const Buffers& b, const DevParams& p, const Tuning& t
 // that serves the scene, 0 for none (the per-phase kernels).
 cudaError_t small_step_setup(int device, const DevParams& p, Buffers* b);
 int small_step_form(const Buffers& b, const DevParams& p);
+bool small_step_waits(int form);  // whether its barrier can give up (PBF_ERRBIT_TIMEOUT)
 cudaError_t launch_step_small(const Buffers& b, const DevParams& p, int form, int cur, float dt, int iters,
                               bool keep_pred, cudaStream_t s);
 cudaError_t launch_resort(const Buffers& b, const DevParams& p, const Tuning& t, int cur,

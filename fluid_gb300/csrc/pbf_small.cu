@@ -13,7 +13,10 @@
 // Barrier: a counter that every block adds one to; thread 0 of a block waits until the count
 // reaches the stage's target. A wait gives up after a bounded number of reads, sets
 // PBF_ERRBIT_TIMEOUT and returns (the launch is cooperative, so every block is resident and a
-// wait ends). The last block to leave sets the counter back to zero.
+// wait ends). No block passes a barrier that another one has not reached, so a launch that gives up
+// leaves its memory in bounds, but the counter and the cell counts stay as they are: a launch that
+// finds the bit set returns before its first write. The last block to leave sets the counter back
+// to zero.
 #include <cstdint>
 
 #include "pbf_device.cuh"
@@ -29,7 +32,7 @@ constexpr int kOwnEntries = 64;                        // list entries of a part
 constexpr int kMaxSums = 5;                            // accumulators of one walk over a list
 constexpr int kRounds = 4;                             // pairs a lane evaluates between two exchanges
 constexpr uint32_t kDirectTiles = 16;                  // tiles up to which a block sums the counts before its own
-constexpr int kMaxPolls = 1 << 22;
+constexpr unsigned kMaxPolls = 1u << 22;             // reads of the barrier's counter (Buffers::wait_reads 0)
 constexpr uint32_t kClusterBlocks = 16;
 
 struct SmallStep {
@@ -43,23 +46,23 @@ struct SmallStep {
   uint32_t* words;
   const SceneDesc* scenes;
   unsigned *err, *bar;
+  unsigned polls;
   uint32_t m;
   int n, iters;
   float dt, inv_dt, one;
 };
 
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, unsigned* err) {
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned target, unsigned polls, unsigned* err) {
   __shared__ bool passed;
   __syncthreads();
   if (threadIdx.x == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-    int left = kMaxPolls;
     unsigned seen;
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-    } while (seen < target && --left > 0);
-    passed = left > 0;
-    if (left <= 0) atomicOr(err, PBF_ERRBIT_TIMEOUT);
+    } while (seen < target && --polls > 0);
+    passed = seen >= target;
+    if (!passed) atomicOr(err, PBF_ERRBIT_TIMEOUT);
   }
   __syncthreads();
   return passed;
@@ -224,7 +227,7 @@ __global__ void __launch_bounds__(T, 512 / T) k_step_small(const __grid_constant
 #define PBF_GRID_BARRIER()                                       \
   if constexpr (CLUSTER)                                         \
     cluster_barrier();                                           \
-  else if (!grid_barrier(A.bar, target += G, A.err))             \
+  else if (!grid_barrier(A.bar, target += G, A.polls, A.err))             \
     return
 
   // prediction (particles.cpp:175-183, 87-132) and cell counts
@@ -237,6 +240,12 @@ __global__ void __launch_bounds__(T, 512 / T) k_step_small(const __grid_constant
   if (live) {
     x4 = A.pos_a[i];
     id = A.id_a[i];
+  }
+  // a step before gave up: its barrier and counts are unusable (read beside the particles)
+  if constexpr (!CLUSTER) {
+    if (__syncthreads_or(static_cast<int>(__ldcg(A.err) & PBF_ERRBIT_TIMEOUT))) return;
+  }
+  if (live) {
     const SceneDesc& sc = A.scenes[scene_of_slot(x4)];
     const float3 x = f3(x4);
     collide<false, false>(x, d, predict_delta(A.vel_a[i], P, A.dt), true, sc, P);
@@ -607,6 +616,8 @@ int small_step_form(const Buffers& b, const DevParams& P) {
   return form_for(b.n, b.n_cells, static_cast<size_t>(b.small_sms));
 }
 
+bool small_step_waits(int form) { return form != 0 && !pick(form, true).cluster; }
+
 cudaError_t launch_step_small(const Buffers& b, const DevParams& P, int form, int cur, float dt, int iters,
                               bool keep_pred, cudaStream_t s) {
   const int A = cur, B = 1 - cur;
@@ -633,6 +644,7 @@ cudaError_t launch_step_small(const Buffers& b, const DevParams& P, int form, in
   a.scenes = b.scenes;
   a.err = b.err;
   a.bar = b.grid_bar;
+  a.polls = b.wait_reads ? b.wait_reads : kMaxPolls;
   a.m = b.n_cells;
   a.n = static_cast<int>(b.n);
   a.iters = iters;

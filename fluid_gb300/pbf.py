@@ -20,7 +20,7 @@ from .params import CParams, PbfParams
 LIB_PATH = Path(os.environ.get("PBF_LIB") or Path(__file__).resolve().parent / "_lib" / "libpbf.so")
 
 PBF_OK = 0
-ABI_VERSION = 6  # PBF_ABI_VERSION of include/pbf.h that these declarations follow
+ABI_VERSION = 7  # PBF_ABI_VERSION of include/pbf.h that these declarations follow
 STATUS = {0: "PBF_OK", 1: "PBF_ERR_INVALID", 2: "PBF_ERR_CUDA", 3: "PBF_ERR_TIMEOUT",
           4: "PBF_ERR_NONFINITE", 5: "PBF_ERR_CAPACITY", 6: "PBF_ERR_NOMEM"}
 
@@ -105,6 +105,7 @@ def _declare(L):
         "pbf_step": (st, [P, ctypes.c_double, ctypes.c_int]),
         "pbf_step_async": (st, [P, ctypes.c_double, ctypes.c_int]),
         "pbf_sync": (st, [P]),
+        "pbf_set_wait_limit": (st, [P, ctypes.c_uint32]),
         "pbf_stream": (P, [P]),
         "pbf_get_positions": (st, [P, P]),
         "pbf_get_velocities": (st, [P, P]),
@@ -263,6 +264,10 @@ class Simulator:
 
     def sync(self):
         self._check(lib().pbf_sync(self._h))
+
+    def set_wait_limit(self, reads: int = 0):
+        """pbf_set_wait_limit: when a wait inside a small scene's step gives up (0: the default)."""
+        self._check(lib().pbf_set_wait_limit(self._h, int(reads)))
 
     @property
     def stream(self) -> int:

@@ -26,7 +26,7 @@
 extern "C" {
 #endif
 
-#define PBF_ABI_VERSION 6
+#define PBF_ABI_VERSION 7
 
 #if defined(__GNUC__)
 #define PBF_API __attribute__((visibility("default")))
@@ -136,6 +136,11 @@ PBF_API pbf_status pbf_step(pbf_handle* h, double dt, int nsteps);
  * (no error check); pbf_sync waits and reports device-side errors. */
 PBF_API pbf_status pbf_step_async(pbf_handle* h, double dt, int nsteps);
 PBF_API pbf_status pbf_sync(pbf_handle* h);
+/* Reads of the barrier after which a wait inside a small scene's step gives up (0: 4 million, some
+ * seconds; scenes of up to 1,024 particles wait in hardware, without a limit). The step then ends
+ * with PBF_ERR_TIMEOUT and the handle stays failed: its state is neither the old nor the new one,
+ * and calls that step, read or reorder it return PBF_ERR_TIMEOUT. Drops captured graphs. */
+PBF_API pbf_status pbf_set_wait_limit(pbf_handle* h, uint32_t reads);
 /* The handle's cudaStream_t (as void*), for ordering and event timing. */
 PBF_API void* pbf_stream(pbf_handle* h);
 
