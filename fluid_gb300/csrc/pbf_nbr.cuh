@@ -292,7 +292,7 @@ __device__ __forceinline__ void nbr_build_warp(NbrWarp& S, int i, const float4* 
         const unsigned rel = at - 32u * static_cast<unsigned>(c);
         const unsigned begun = __reduce_or_sync(full, (cnt && rel < 32u) ? 1u << rel : 0u);  // rows that begin here
         float4 xj;
-        xj.x = INFINITY;  // no candidate: no hit
+        xj.x = NAN;  // no candidate: no hit, also for an h2 beyond FP32's range (infinity)
         if (k < T) {
           const int2 de = S.de[rows + __popc(begun & upto)];
           const int j = k + de.x;
