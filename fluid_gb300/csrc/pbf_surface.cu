@@ -184,6 +184,18 @@ __global__ void k_surf_cells(const uint32_t* __restrict__ cell_start, const Scen
   any[c] = some ? 1 : 0;
 }
 
+// Whether the lanes of a box [lo, hi] walk the rows around all of it (density_together), or each
+// lane those around its own point: a wide box holds many candidates that are near few of its
+// points, and each lane would read all of them. A surface of 1M particles with cubes of h (a box of
+// 1 cell): 250 us together, 290 each; cubes of 1.5 h 257 and 189, 2 h 281 and 171, 4 h 485 and 168,
+// 40 h 18,900 and 97.
+constexpr float kTogetherCells = 1.25f;
+__device__ __forceinline__ bool walk_together(const float3 lo, const float3 hi, const SceneDesc& sc,
+                                              const DevParams& P) {
+  const float w = fmaxf(fmaxf(hi.x - lo.x, hi.y - lo.y), hi.z - lo.z) * P.inv_cell;
+  return w <= kTogetherCells && in_grid(lo, sc, P.inv_cell) && in_grid(hi, sc, P.inv_cell);
+}
+
 // The field, z fastest (the cubes' loop order, so the passes over the cubes read it in lines). 8
 // lanes take a block of 2 x 2 x 2 corners and walk its candidates together: with a candidate list
 // of its own per lane the pass is bound by the L1 data pipe (a load of 32 lanes touches about 20
@@ -209,9 +221,9 @@ __global__ void __launch_bounds__(128) k_surf_density(const float4* __restrict__
   const bool near = live && any[cell_key(cell_of(p, sc, P.inv_cell), sc)] != 0;
   float v = 0.f;
   if ((__ballot_sync(0xffffffffu, near) >> (lane & 24)) & 0xffu) {
-    if (in_grid(lo, sc, P.inv_cell) && in_grid(hi, sc, P.inv_cell))
+    if (walk_together(lo, hi, sc, P))
       v = P.poly6_c * density_together(p, lo, hi, pos, cell_start, sc, P);
-    else
+    else if (near)
       v = density_at_point(p, pos, cell_start, sc, P);
   }
   if (live) field[(static_cast<uint32_t>(i) * ny + j) * nz + k] = v;
@@ -460,9 +472,8 @@ __global__ void __launch_bounds__(128) k_surf_vnormals(const float* __restrict__
   float3 p = x;
   set3(p, q >> 1, (q & 1) ? cmp3(hi, q >> 1) : cmp3(lo, q >> 1));
   const SceneDesc& sc = scenes[0];
-  const bool together = in_grid(lo, sc, P.inv_cell) && in_grid(hi, sc, P.inv_cell);
-  const float v = together ? density_together(p, lo, hi, pos, cell_start, sc, P)
-                           : density_sum_at(p, pos, cell_start, sc, P);
+  const float v = walk_together(lo, hi, sc, P) ? density_together(p, lo, hi, pos, cell_start, sc, P)
+                                               : density_sum_at(p, pos, cell_start, sc, P);
   __syncwarp();
   // lanes 0, 2, 4: the density below less the one above, the former not rounded first
   const float d = __fmaf_rn(P.poly6_c, v, -__fmul_rn(P.poly6_c, __shfl_down_sync(0xffffffffu, v, 1)));
