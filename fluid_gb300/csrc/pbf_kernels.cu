@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(BLOCK, 1152 / BLOCK) k_nbr_build(const float4*
                                                      unsigned* __restrict__ err, DevParams P, float one, int n) {
   chain_begin();
   extern __shared__ uint4 nbr_smem[];
-  nbr_build_warp<true>(reinterpret_cast<NbrWarp*>(nbr_smem)[threadIdx.x >> 5],
+  nbr_build_warp<true, true>(reinterpret_cast<NbrWarp*>(nbr_smem)[threadIdx.x >> 5],
                        static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x), xs, pos, cell_start, scenes, hdr,
                        words, err, P, one, n);
 }

@@ -17,8 +17,9 @@ __device__ __forceinline__ T ld(const T* p) {
   return NC ? __ldg(p) : *p;
 }
 
-// One thread scans one particle's candidates: for the warps whose slots lie in many rows, or
-// whose candidate windows exceed the shared tables of the warp scan (k_nbr_build). Each of the
+// One thread scans one particle's candidates: for the warps whose slots lie far apart (in many rows,
+// or along them), that are next to a cell too large to be sorted, or whose list offsets pass their 14
+// bits; in the whole-step kernel also where windows exceed the shared tables. Each of the
 // 9 candidate rows (3 z-slabs x 3 y-rows) is skipped when its cells lie beyond h in y/z, and
 // otherwise trimmed in x to the cells that reach [x - w, x + w], w = sqrt(h^2 - d_yz^2): about
 // 20 of the 27 cells on average. Within the trimmed row (sorted by x, see k_cellrank) only
@@ -148,7 +149,12 @@ __device__ __noinline__ void nbr_scan_thread(int i, const float4* xs, const floa
 // rows left untrimmed (193 us).
 constexpr int kNbrWords = 14;    // ballot words per slot: at most 448 candidates a group
 constexpr int kNbrEntries = 1408;  // candidates of the groups of a round, each group's rounded up to 32
-constexpr int kNbrGroups = 6;    // more groups (slots scattered over rows): the thread scan
+// The thread scan takes the warps of more groups than the tables hold (slots scattered over rows),
+// and those whose groups' windows are so many cells long in all that a lane has few candidates of
+// its own in them: 0.13 particles a cell 33.8 us with the group scan, 30.0 with the thread scan; 0.5
+// a cell (80 to 100 cells) 96 and 110; rest spacing has about 18 cells, 1 particle a cell 55.
+constexpr int kNbrGroups = 6;
+constexpr int kNbrSpan = 160;
 struct NbrWarp {
   uint32_t mask[kNbrWords][32];   // [turn][slot]: the turn's 32 candidates within h of the slot
   float4 txy[16];                 // slots 2p and 2p + 1: -x, -x, -y, -y
@@ -163,18 +169,24 @@ struct NbrWarp {
                                    // by lanes past their hits
 };
 
-// Builds the list of slot i (lane's slot of a warp of 32 consecutive ones; i >= n: none). S: the
-// warp's shared tables. one: 1, unknown to the compiler.
-template <bool NC>
-__device__ __forceinline__ void nbr_build_warp(NbrWarp& S, int i, const float4* xs, const float4* pos,
-                                               const uint32_t* cell_start, const SceneDesc* __restrict__ scenes,
-                                               uint4* hdr, uint32_t* words, unsigned* err, const DevParams& P,
-                                               float one, int n) {
+enum NbrResult { kNbrDone, kNbrParts, kNbrThread };  // a warp's lists: made; left to PARTS; to the thread scan
+
+// PARTS: a group with more candidates than the words hold is read in pieces, each appending to the
+// lists of the pieces before (16-bit stores; clumps of 2.6 times the rest spacing's density and more:
+// 262k particles at 93 neighbours 199 -> 154 us, at 114 neighbours 405 -> 254, by the thread scan
+// before). A code of its own, behind the first try, because its registers cost the common case 0.5%.
+template <bool NC, bool PARTS>
+__device__ __forceinline__ NbrResult nbr_build_lists(NbrWarp& S, int i, const float4* xs, const float4* pos,
+                                                     const uint32_t* cell_start, const SceneDesc* __restrict__ scenes,
+                                                     uint4* hdr, uint32_t* words, unsigned* err, const DevParams& P,
+                                                     float one, int n) {
   const unsigned full = 0xffffffffu;
   const int lane = static_cast<int>(lane_id());
   const bool live = i < n;
   const unsigned alive = __ballot_sync(full, live);  // a prefix of the lanes
-  if (!alive) return;
+  if (!alive) return kNbrDone;
+  const unsigned upto = lane == 31 ? full : ((2u << lane) - 1u);
+  const float2 ones = make_float2(one, one);  // 1, unknown to the compiler
   const float4 xi = live ? xs[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   const int scn = live ? scene_of_slot(pos[i]) : 0;
   uint32_t row0 = 0xffffffffu;
@@ -187,86 +199,87 @@ __device__ __forceinline__ void nbr_build_warp(NbrWarp& S, int i, const float4* 
   const uint32_t prev = __shfl_up_sync(full, row0, 1);
   const bool head = live && ((lane & 7) == 0 || prev != row0);
   const unsigned heads = __ballot_sync(full, head);
-  const int ngroups = __popc(heads);
-  const unsigned upto = lane == 31 ? full : ((2u << lane) - 1u);
-  bool ok = ngroups <= kNbrGroups;
-  if (ok) {
-    if (head) S.first[__popc(heads & upto) - 1] = lane;
-    if (lane == 0) S.first[ngroups] = __popc(alive);
-    const int p2 = lane >> 1, q2 = lane & 1;
-    reinterpret_cast<float*>(&S.txy[p2])[q2] = -xi.x;
-    reinterpret_cast<float*>(&S.txy[p2])[2 + q2] = -xi.y;
-    reinterpret_cast<float*>(&S.tz[p2])[q2] = -xi.z;
-    __syncwarp();
-    // The candidate ranges, one (group, row) per lane and round: whole cells, trimmed in x to the
-    // reach of the group's slots, h plus a margin of 1e-3 cell (NaN coordinates leave a range
-    // untrimmed).
-    const float W = (sqrtf(P.h2) * P.inv_cell + 1e-3f) * (1.0f / P.inv_cell);
-    for (int base = 0; base < 9 * ngroups; base += 32) {
-      const int q = base + lane;
-      const bool act = q < 9 * ngroups;
-      const int s = act ? q / 9 : 0, r = act ? q - 9 * s : 0;
-      const int f = S.first[s], l = S.first[s + 1] - 1;
-      const int cy = __shfl_sync(full, cc.y, f), cz = __shfl_sync(full, cc.z, f);
-      const int cxa = __shfl_sync(full, cc.x, f), cxb = __shfl_sync(full, cc.x, l);
-      const float xa = __shfl_sync(full, xi.x, f), xb = __shfl_sync(full, xi.x, l);
-      const int gs = __shfl_sync(full, scn, f);
-      if (act) {
-        const SceneDesc& sc = scenes[gs];
-        const int d0 = sc.dim[0], d1 = sc.dim[1], d2 = sc.dim[2];
-        const int g = r / 3, z = cz + g - 1, y = cy + (r - 3 * g) - 1;
-        uint32_t lo = 0, lo2 = 0, gb = 0;
-        if (z >= 0 && z < d2) {
-          const uint32_t slab = sc.cell_off + static_cast<uint32_t>(z * d1 * d0);
-          const int a = max(cxa - 1, 0), b = min(cxb + 1, d0 - 1);
-          gb = ld<NC>(&cell_start[slab + static_cast<uint32_t>(max(cy - 1, 0) * d0 + a)]);
-          if (y >= 0 && y < d1) {
-            const uint32_t row = slab + static_cast<uint32_t>(y * d0);
-            lo = ld<NC>(&cell_start[row + a]);
-            lo2 = ld<NC>(&cell_start[row + b]);
-            uint32_t hi = ld<NC>(&cell_start[row + a + 1]), hi2 = ld<NC>(&cell_start[row + b + 1]);
-            if (hi2 - lo > static_cast<uint32_t>(kMaxRowCandidates)) ok = false;  // reported by the thread scan
-            while (lo < hi || lo2 < hi2) {  // first x >= xa - W of the first cell; first x > xb + W of the last
-              const uint32_t md = (lo + hi) >> 1, md2 = (lo2 + hi2) >> 1;
-              if (lo < hi) {
-                if (ld<NC>(&xs[md].x) - xa < -W) lo = md + 1; else hi = md;
-              }
-              if (lo2 < hi2) {
-                if (ld<NC>(&xs[md2].x) - xb > W) hi2 = md2; else lo2 = md2 + 1;
-              }
+  const int ng = __popc(heads), group = __popc(heads & upto) - 1;  // groups; the lane's
+  if (!PARTS) {
+    // cells along x of the groups' windows
+    const unsigned above = heads & ~upto;
+    const int last = (above ? __ffs(above) - 1 : __popc(alive)) - 1;
+    const int span = __shfl_sync(full, cc.x, last) - cc.x + 3;
+    if (ng > kNbrGroups || __reduce_add_sync(full, head ? span : 0) > kNbrSpan) return kNbrThread;
+  }
+  if (head) S.first[group] = lane;
+  if (lane == 0) S.first[ng] = __popc(alive);
+  const int p2 = lane >> 1, q2 = lane & 1;
+  reinterpret_cast<float*>(&S.txy[p2])[q2] = -xi.x;
+  reinterpret_cast<float*>(&S.txy[p2])[2 + q2] = -xi.y;
+  reinterpret_cast<float*>(&S.tz[p2])[q2] = -xi.z;
+  __syncwarp();
+  // The candidate ranges, one (group, row) per lane and round: whole cells, trimmed in x to the
+  // reach of the group's slots, h plus a margin of 1e-3 cell (NaN coordinates leave a range
+  // untrimmed).
+  bool ok = true, room = true;
+  const float W = (sqrtf(P.h2) * P.inv_cell + 1e-3f) * (1.0f / P.inv_cell);
+  for (int base = 0; base < 9 * ng; base += 32) {
+    const int q = base + lane;
+    const bool act = q < 9 * ng;
+    const int s = act ? q / 9 : 0, r = act ? q - 9 * s : 0;
+    const int f = S.first[s], l = S.first[s + 1] - 1;
+    const int cy = __shfl_sync(full, cc.y, f), cz = __shfl_sync(full, cc.z, f);
+    const int cxa = __shfl_sync(full, cc.x, f), cxb = __shfl_sync(full, cc.x, l);
+    const float xa = __shfl_sync(full, xi.x, f), xb = __shfl_sync(full, xi.x, l);
+    const int gs = __shfl_sync(full, scn, f);
+    if (act) {
+      const SceneDesc& sc = scenes[gs];
+      const int d0 = sc.dim[0], d1 = sc.dim[1], d2 = sc.dim[2];
+      const int g = r / 3, z = cz + g - 1, y = cy + (r - 3 * g) - 1;
+      uint32_t lo = 0, lo2 = 0, gb = 0;
+      if (z >= 0 && z < d2) {
+        const uint32_t slab = sc.cell_off + static_cast<uint32_t>(z * d1 * d0);
+        const int a = max(cxa - 1, 0), b = min(cxb + 1, d0 - 1);
+        gb = ld<NC>(&cell_start[slab + static_cast<uint32_t>(max(cy - 1, 0) * d0 + a)]);
+        if (y >= 0 && y < d1) {
+          const uint32_t row = slab + static_cast<uint32_t>(y * d0);
+          lo = ld<NC>(&cell_start[row + a]);
+          lo2 = ld<NC>(&cell_start[row + b]);
+          uint32_t hi = ld<NC>(&cell_start[row + a + 1]), hi2 = ld<NC>(&cell_start[row + b + 1]);
+          if (hi2 - lo > static_cast<uint32_t>(kMaxRowCandidates)) ok = false;  // reported by the thread scan
+          while (lo < hi || lo2 < hi2) {  // first x >= xa - W of the first cell; first x > xb + W of the last
+            const uint32_t md = (lo + hi) >> 1, md2 = (lo2 + hi2) >> 1;
+            if (lo < hi) {
+              if (ld<NC>(&xs[md].x) - xa < -W) lo = md + 1; else hi = md;
+            }
+            if (lo2 < hi2) {
+              if (ld<NC>(&xs[md2].x) - xb > W) hi2 = md2; else lo2 = md2 + 1;
             }
           }
         }
-        const uint32_t cnt = lo2 > lo ? lo2 - lo : 0u;
-        if (cnt && lo2 - 1 - gb > kOffsetMask) ok = false;
-        S.row[q] = make_uint4(lo, cnt, (static_cast<uint32_t>(g) << kOffsetBits) - gb, 0u);
-        if (r == 3 * g + 1) S.gb[3 * s + g] = gb;
       }
+      const uint32_t cnt = lo2 > lo ? lo2 - lo : 0u;
+      if (cnt && lo2 - 1 - gb > kOffsetMask) ok = false;
+      S.row[q] = make_uint4(lo, cnt, (static_cast<uint32_t>(g) << kOffsetBits) - gb, 0u);
+      if (r == 3 * g + 1) S.gb[3 * s + g] = gb;
     }
-    __syncwarp();
-    uint32_t t = 0;  // lane s: group s
-    if (lane < ngroups) {
-#pragma unroll
-      for (int r = 0; r < 9; ++r) t += min(S.row[9 * lane + r].y, 32u * kNbrWords + 1u);
-    }
-    if (lane < ngroups) {
-      S.cand[lane] = static_cast<int>(t);
-      ok = ok && t <= 32u * kNbrWords;
-    }
-  }
-  if (!__all_sync(full, ok)) {
-    if (live) nbr_scan_thread<NC>(i, xs, pos, cell_start, scenes, hdr, words, err, P, n);
-    return;
   }
   __syncwarp();
-  const float2 ones = make_float2(one, one);  // 1, unknown to the compiler
-  int s = 0;
+  if (lane < ng) {  // lane s: group s
+    uint32_t t = 0;
+#pragma unroll
+    for (int r = 0; r < 9; ++r) t += S.row[9 * lane + r].y;
+    S.cand[lane] = static_cast<int>(t);
+    if (!PARTS) room = t <= 32u * kNbrWords;
+  }
+  if (!__all_sync(full, ok)) return kNbrThread;
+  if (!PARTS && !__all_sync(full, room)) return kNbrParts;
+  __syncwarp();
+  int s = 0, turn0 = 0;  // the next group and its first turn: a group beyond the words goes in pieces
   do {  // rounds of as many groups as the entries have room for (dense windows: fewer than all)
-    const int s_begin = s;
+    const int s_begin = s, t_begin = turn0;
     int used = 0;
-    for (; s < ngroups && used + S.cand[s] <= kNbrEntries; ++s) {
+    for (; s < ng; ++s) {
+      const int rest = S.cand[s] - 32 * turn0;
+      const int T = min(rest, 32 * kNbrWords), eoff = used;
+      if (used + T > kNbrEntries) break;
       const int f = S.first[s], l = S.first[s + 1] - 1;
-      const int T = S.cand[s], eoff = used;
       used += (T + 31) & ~31;
       if (lane == 0) S.eoff[s] = eoff;
       // lane r < 9: row r's range in the flat list; the non-empty rows in order in S.de
@@ -278,7 +291,7 @@ __device__ __forceinline__ void nbr_build_warp(NbrWarp& S, int i, const float4* 
         const uint32_t v = __shfl_up_sync(full, incl, o);
         if (lane >= o) incl += v;
       }
-      const uint32_t at = incl - cnt;
+      const uint32_t at = incl - cnt - 32u * static_cast<unsigned>(turn0);  // less the turns before
       const unsigned some = __ballot_sync(full, cnt > 0);
       if (cnt) S.de[__popc(some & upto) - 1] = make_int2(static_cast<int>(start - at), static_cast<int>(row.z));
       // the 8 slots of the group's eighth, in pairs
@@ -286,7 +299,8 @@ __device__ __forceinline__ void nbr_build_warp(NbrWarp& S, int i, const float4* 
       const uint32_t ta = static_cast<uint32_t>(__cvta_generic_to_shared(&S.txy[(f & ~7) >> 1]));
       const uint32_t tb = static_cast<uint32_t>(__cvta_generic_to_shared(&S.tz[(f & ~7) >> 1]));
       __syncwarp();
-      int rows = -1;  // non-empty rows begun before the turn, less one
+      // non-empty rows begun before the turn, less one
+      int rows = __popc(__ballot_sync(full, cnt > 0 && static_cast<int>(at) < 0)) - 1;
       for (int c = 0; 32 * c < T; ++c) {
         const int k = 32 * c + lane;
         const unsigned rel = at - 32u * static_cast<unsigned>(c);
@@ -331,39 +345,43 @@ __device__ __forceinline__ void nbr_build_warp(NbrWarp& S, int i, const float4* 
       __syncwarp();
       // the own slot, a hit at distance 0 in the middle row
       const uint32_t s4 = __shfl_sync(full, start, 4), a4 = __shfl_sync(full, at, 4), c4 = __shfl_sync(full, cnt, 4);
-      const uint32_t own = static_cast<uint32_t>(i) - s4;
-      if (lane >= f && lane <= l && own < c4) {
-        const uint32_t k = a4 + own;
-        S.mask[k >> 5][lane] &= ~(1u << (k & 31u));
-      }
+      const uint32_t own = static_cast<uint32_t>(i) - s4, k4 = a4 + own;
+      if (lane >= f && lane <= l && own < c4 && k4 < static_cast<uint32_t>(T))
+        S.mask[k4 >> 5][lane] &= ~(1u << (k4 & 31u));
       __syncwarp();
+      if (PARTS && T < rest) {  // the rest of its candidates in the rounds after
+        turn0 += kNbrWords;
+        break;
+      }
+      turn0 = 0;
     }
     // lists: the lanes take their hits in order, each the next set bit of its words (words
     // without a hit are skipped by the mask of the others), all at the same entry index
-    int total = 0;
+    int total = 0, have = 0;
     unsigned words_left = 0;
-    const int group = __popc(heads & upto) - 1;
-    const bool mine = live && group >= s_begin && group < s;
+    const bool mine = live && group >= s_begin && group < s + (turn0 ? 1 : 0);
     int own_at = 0;
     if (mine) {
       own_at = S.eoff[group];
-      const int nw = (S.cand[group] + 31) >> 5;
+      const int skip = group == s_begin ? t_begin : 0;
+      const int nw = min((S.cand[group] - 32 * skip + 31) >> 5, kNbrWords);
+      if (skip) have = nbr_total(hdr[i]);
       for (int c = 0; c < nw; ++c) {
         const uint32_t m = S.mask[c][lane];
         total += __popc(m);
         words_left |= m ? 1u << c : 0u;
       }
     }
-    const int cap = P.max_words * 2;
-    if (total > cap) {
+    const int room = P.max_words * 2 - have;
+    if (total > room) {
       atomicOr(err, PBF_ERRBIT_NEIGHBOR_CAPACITY);
-      total = cap;
+      total = room;
     }
     if (mine) {
       const uint32_t g0 = S.gb[3 * group];
       // the slab bases relative to slab 0's, less the tag bits (nbr_decode)
       hdr[i] = make_uint4(g0, S.gb[3 * group + 1] - g0 - (1u << kOffsetBits),
-                          S.gb[3 * group + 2] - g0 - (2u << kOffsetBits), static_cast<uint32_t>(total));
+                          S.gb[3 * group + 2] - g0 - (2u << kOffsetBits), static_cast<uint32_t>(have + total));
     }
     const int most = __reduce_max_sync(full, total);
     uint4* out = reinterpret_cast<uint4*>(words) + i;
@@ -382,12 +400,38 @@ __device__ __forceinline__ void nbr_build_warp(NbrWarp& S, int i, const float4* 
         q[u] = ent[(__ffs(m) - 1) & 31];
         m &= m - 1;
       }
-      if (k < total)
-        out[static_cast<size_t>(k >> 3) * n] =
-            make_uint4(q[0] | q[1] << 16, q[2] | q[3] << 16, q[4] | q[5] << 16, q[6] | q[7] << 16);
+      if (!PARTS || t_begin == 0) {
+        if (k < total)
+          out[static_cast<size_t>(k >> 3) * n] =
+              make_uint4(q[0] | q[1] << 16, q[2] | q[3] << 16, q[4] | q[5] << 16, q[6] | q[7] << 16);
+      } else {  // behind the entries of the pieces before
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int e = have + k + u;
+          if (k + u < total)
+            reinterpret_cast<uint16_t*>(out + static_cast<size_t>(e >> 3) * n)[e & 7] = static_cast<uint16_t>(q[u]);
+        }
+      }
     }
     __syncwarp();
-  } while (s < ngroups);
+  } while (s < ng);
+  return kNbrDone;
+}
+
+// Builds the list of slot i (lane's slot of a warp of 32 consecutive ones; i >= n: none). S: the
+// warp's shared tables. one: 1, unknown to the compiler. DENSE: groups beyond the words in pieces
+// (false: by the thread scan, for a kernel that has no room for the code).
+template <bool NC, bool DENSE>
+__device__ __forceinline__ void nbr_build_warp(NbrWarp& S, int i, const float4* xs, const float4* pos,
+                                               const uint32_t* cell_start, const SceneDesc* __restrict__ scenes,
+                                               uint4* hdr, uint32_t* words, unsigned* err, const DevParams& P,
+                                               float one, int n) {
+  NbrResult r = nbr_build_lists<NC, false>(S, i, xs, pos, cell_start, scenes, hdr, words, err, P, one, n);
+  if (r == kNbrDone) return;
+  if (DENSE && r == kNbrParts)
+    nbr_build_lists<NC, true>(S, i, xs, pos, cell_start, scenes, hdr, words, err, P, one, n);
+  else if (i < n)
+    nbr_scan_thread<NC>(i, xs, pos, cell_start, scenes, hdr, words, err, P, n);
 }
 
 }  // namespace pbf

@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(T, 512 / T) k_step_small(const __grid_constant
     }
   }
   if (front)
-    nbr_build_warp<false>(reinterpret_cast<NbrWarp*>(work)[tid >> 5], i, A.xs0, A.pos_b, A.start, A.scenes, A.hdr,
+    nbr_build_warp<false, false>(reinterpret_cast<NbrWarp*>(work)[tid >> 5], i, A.xs0, A.pos_b, A.start, A.scenes, A.hdr,
                           A.words, A.err, P, A.one, n);
   if constexpr (CLUSTER)
     cluster_barrier();  // every block has its copies before another one stores into them
