@@ -238,7 +238,7 @@ pbf_status Handle::alloc_all() {
                        "cudaMemsetAsync");  // the scan's ticket word (after the tile sums) starts at zero
   if (st == PBF_OK) st = cuda(cudaMemsetAsync(b.cell_count, 0, sizeof(uint32_t) * b.n_cells, stream), "cudaMemsetAsync");
   b.grid_bar = b.err + 1;
-  if (st == PBF_OK) st = cuda(small_step_setup(device, dp, &b), "occupancy");
+  if (st == PBF_OK) small_step_setup(device, dp, &b);
   if (st == PBF_OK && small_step_waits(small_step_form(b, dp))) {
     // the second buffers hold valid indexes before their first step: what follows a step that gave
     // up (usable) reads them
@@ -1522,6 +1522,11 @@ pbf_status pbf_reset_phase_times(pbf_handle* hh) {
 }
 
 size_t pbf_size(const pbf_handle* hh) { return hh ? reinterpret_cast<const Handle*>(hh)->b.n : 0; }
+
+int pbf_step_form(const pbf_handle* hh) {
+  const Handle* h = reinterpret_cast<const Handle*>(hh);
+  return h ? pbf::small_step_form(h->b, h->dp) : 0;
+}
 
 int pbf_num_scenes(const pbf_handle* hh) { return hh ? reinterpret_cast<const Handle*>(hh)->b.n_scenes : 0; }
 

@@ -116,7 +116,7 @@ struct Buffers {
   unsigned int* err = nullptr;     // sticky PBF_ERRBIT_* word, then the three of grid_bar
   unsigned int* grid_bar = nullptr;  // counters, zero between launches: the whole-step kernel's barrier and the
                                      // blocks that left it, the statistics pass's ticket
-  int small_sms = 0;                 // SMs for the whole-step kernel (0: not used)
+  int small_form = 0;                // form of the whole-step kernel (0: not used)
   unsigned wait_reads = 0;           // reads after which a wait inside a step gives up (0: 4 million)
   float* io = nullptr;             // (n, 3) staging for host/device packed transfers
   float* io2 = nullptr;
@@ -227,10 +227,10 @@ cudaError_t launch_adjoint(const Buffers& b, const DevParams& p, const Tuning& t
                            const Tape& tape, const float* gx_out, const float* gv_out, float* gx_in,
                            float* gv_in, double* g_rho0, cudaStream_t s);
 // ---- the whole step in one cooperative launch (pbf_small.cu): same results ----
-// small_step_setup: b->small_sms, the device's SM count when the handle's scenes take the launch and
-// the device can, else 0 (n, n_cells and p.scorr_n do not change afterwards). small_step_form: the form
-// that serves the scene, 0 for none (the per-phase kernels).
-cudaError_t small_step_setup(int device, const DevParams& p, Buffers* b);
+// small_step_setup: b->small_form, the form that serves the handle's scenes and that the device takes, 0
+// for none: the per-phase kernels (n, n_cells and p.scorr_n do not change afterwards). small_step_form:
+// the form a step takes (with the colliders the handle has now).
+void small_step_setup(int device, const DevParams& p, Buffers* b);
 int small_step_form(const Buffers& b, const DevParams& p);
 bool small_step_waits(int form);  // whether its barrier can give up (PBF_ERRBIT_TIMEOUT)
 cudaError_t launch_step_small(const Buffers& b, const DevParams& p, int form, int cur, float dt, int iters,

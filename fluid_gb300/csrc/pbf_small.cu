@@ -21,19 +21,19 @@
 
 #include "pbf_device.cuh"
 #include "pbf_nbr.cuh"
+#include "pbf_small_form.h"
 #include "pbf_step.cuh"
 
 namespace pbf {
 namespace {
 
-constexpr uint32_t kScanTile = 1024;                   // cells; scan_tmp has an entry per tile
+constexpr uint32_t kScanTile = kSmallTile;             // cells; scan_tmp has an entry per tile
 constexpr uint32_t kMaxSortedCell = 4096;              // larger cells keep the atomic order (as k_cellsort_big)
 constexpr int kOwnEntries = 64;                        // list entries of a particle kept on chip
 constexpr int kMaxSums = 5;                            // accumulators of one walk over a list
 constexpr int kRounds = 4;                             // pairs a lane evaluates between two exchanges
 constexpr uint32_t kDirectTiles = 16;                  // tiles up to which a block sums the counts before its own
 constexpr unsigned kMaxPolls = 1u << 22;             // reads of the barrier's counter (Buffers::wait_reads 0)
-constexpr uint32_t kClusterBlocks = 16;
 
 struct SmallStep {
   const float4 *pos_a, *vel_a;
@@ -531,28 +531,27 @@ Kernel pick_kernel(bool n4) {
 }
 struct Form {
   Kernel kernel;
-  uint32_t threads, per_block;  // threads and particles of a block
+  SmallFormSize size;
   size_t smem;
-  bool cluster;
 };
 Form pick(int form, bool n4) {
+  const SmallFormSize& z = kSmallForm[form];
   switch (form) {
-    case 1: return Form{pick_kernel<512, 8, true>(n4), 512, 64, small_smem<512, 8, true>(), true};
-    case 2: return Form{pick_kernel<256, 8, false>(n4), 256, 32, small_smem<256, 8, false>(), false};
-    case 3: return Form{pick_kernel<128, 1, false>(n4), 128, 128, small_smem<128, 1, false>(), false};
-    default: return Form{pick_kernel<256, 1, false>(n4), 256, 256, small_smem<256, 1, false>(), false};
+    case 1: return Form{pick_kernel<512, 8, true>(n4), z, small_smem<512, 8, true>()};
+    case 2: return Form{pick_kernel<256, 8, false>(n4), z, small_smem<256, 8, false>()};
+    case 3: return Form{pick_kernel<128, 1, false>(n4), z, small_smem<128, 1, false>()};
+    default: return Form{pick_kernel<256, 1, false>(n4), z, small_smem<256, 1, false>()};
   }
 }
-constexpr int kForms = 4;
 
 void set_config(const Form& f, uint32_t blocks, cudaStream_t s, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
   *cfg = cudaLaunchConfig_t{};
   cfg->gridDim = dim3(blocks);
-  cfg->blockDim = dim3(f.threads);
+  cfg->blockDim = dim3(f.size.threads);
   cfg->dynamicSmemBytes = f.smem;
   cfg->stream = s;
   *at = cudaLaunchAttribute{};
-  if (f.cluster) {
+  if (f.size.cluster) {
     at->id = cudaLaunchAttributeClusterDimension;
     at->val.clusterDim.x = blocks;
     at->val.clusterDim.y = at->val.clusterDim.z = 1;
@@ -564,59 +563,47 @@ void set_config(const Form& f, uint32_t blocks, cudaStream_t s, cudaLaunchConfig
   cfg->numAttrs = 1;
 }
 
-// Which form a scene takes; 0: the per-phase kernels. One cluster of 16 blocks of 64 particles, 8
-// lanes each; the same over the grid while two blocks of 32 particles fit on every SM; then one lane
-// a particle with one block on an SM. Steps (us, no statistics) of 8 lanes over the grid /
-// 1 lane / per-phase kernels: 512 particles 59 / 75 / 77, 4,096 65 / 85 / 96, 8,000 73 / 87 / 101;
-// 19k - / 89 / 105, 33k - / 89 / 109; with a second block on some SMs the gain is gone (51k: 115 /
-// 118). 4 lanes a particle over the grid: 8,000 77, 14k 93 (1 lane 89). Handles with collider
-// triangles or spheres keep the per-phase kernels: whether a move meets a triangle's edge turns on
-// the last bit, and the primitives' tests are not pinned to one rounding.
-int form_for(size_t n, size_t n_cells, size_t sms) {
-  const size_t tiles = (n_cells + kScanTile - 1) / kScanTile;
-  for (int form = 1; n > 0 && sms > 0 && form <= kForms; ++form) {
-    const Form f = pick(form, true);
-    const size_t room = f.cluster ? kClusterBlocks : form == 2 ? 2 * sms : sms;
-    if ((n + f.per_block - 1) / f.per_block <= room && tiles <= room) return form;
-  }
-  return 0;
-}
-
-}  // namespace
-
-// Only the kernel that this handle would launch is looked at: each look costs a handle's creation
-// tens of microseconds, and the first one loads the kernel.
-cudaError_t small_step_setup(int device, const DevParams& P, Buffers* b) {
-  b->small_sms = 0;
-  int count = 0, coop = 0, fit = 0;
-  cudaError_t e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device);
-  if (e != cudaSuccess || !coop) return e;
-  const int form = form_for(b->n, b->n_cells, static_cast<size_t>(count));
-  if (form == 0) return cudaSuccess;
-  const Form f = pick(form, P.scorr_n == 4);
-  e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(f.smem));
-  if (e != cudaSuccess) return e;
-  if (f.cluster) {
+// Whether the device takes the form: its launch can be resident. An error is an answer too (a device
+// or a partition of one without clusters of 16 blocks, or with less shared memory): the next form.
+bool takes(int form, bool n4) {
+  const Form f = pick(form, n4);
+  int fit = 0;
+  cudaError_t e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(f.smem));
+  if (e == cudaSuccess && f.size.cluster) {
     e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute at;
     set_config(f, kClusterBlocks, nullptr, &cfg, &at);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fit, f.kernel, &cfg);
-  } else {
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, f.kernel, static_cast<int>(f.threads), f.smem);
-    fit -= form == 2 ? 1 : 0;  // two blocks on an SM
+  } else if (e == cudaSuccess) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, f.kernel, static_cast<int>(f.size.threads), f.smem);
+    fit /= static_cast<int>(f.size.on_sm);
   }
-  if (e == cudaSuccess && fit >= 1) b->small_sms = count;
-  return e;
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e == cudaSuccess && fit >= 1;
 }
 
-int small_step_form(const Buffers& b, const DevParams& P) {
-  if (P.n_mesh > 0 || P.n_sph > 0) return 0;
-  return form_for(b.n, b.n_cells, static_cast<size_t>(b.small_sms));
+}  // namespace
+
+// The kernels are looked at until one is taken, mostly the first: each look costs a handle's creation
+// tens of microseconds, and the first one loads the kernel. Handles with collider triangles or spheres
+// keep the per-phase kernels: whether a move meets a triangle's edge turns on the last bit, and the
+// primitives' tests are not pinned to one rounding.
+void small_step_setup(int device, const DevParams& P, Buffers* b) {
+  int sms = 0, coop = 0;
+  b->small_form = 0;
+  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return;
+  }
+  b->small_form = small_form_for(b->n, b->n_cells, static_cast<size_t>(sms),
+                                 [&](int form) { return takes(form, P.scorr_n == 4); });
 }
 
-bool small_step_waits(int form) { return form != 0 && !pick(form, true).cluster; }
+int small_step_form(const Buffers& b, const DevParams& P) { return P.n_mesh > 0 || P.n_sph > 0 ? 0 : b.small_form; }
+
+bool small_step_waits(int form) { return form != 0 && !kSmallForm[form].cluster; }
 
 cudaError_t launch_step_small(const Buffers& b, const DevParams& P, int form, int cur, float dt, int iters,
                               bool keep_pred, cudaStream_t s) {
@@ -653,7 +640,7 @@ cudaError_t launch_step_small(const Buffers& b, const DevParams& P, int form, in
   a.one = 1.0f;
   const uint32_t tiles = (a.m + kScanTile - 1) / kScanTile;
   const Form f = pick(form, P.scorr_n == 4);
-  const uint32_t need = (static_cast<uint32_t>(b.n) + f.per_block - 1) / f.per_block;
+  const uint32_t need = (static_cast<uint32_t>(b.n) + f.size.per_block - 1) / f.size.per_block;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at;
   set_config(f, need > tiles ? need : tiles, s, &cfg, &at);

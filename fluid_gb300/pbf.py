@@ -142,6 +142,7 @@ def _declare(L):
         "pbf_render_set_scene": (st, [P, P, P, P, sz, P, sz, P, sz]),
         "pbf_render": (st, [P, P, P, P, P, P]),
         "pbf_size": (sz, [P]),
+        "pbf_step_form": (ctypes.c_int, [P]),
         "pbf_num_scenes": (ctypes.c_int, [P]),
         "pbf_last_error": (ctypes.c_char_p, [P]),
     }
@@ -268,6 +269,11 @@ class Simulator:
     def set_wait_limit(self, reads: int = 0):
         """pbf_set_wait_limit: when a wait inside a small scene's step gives up (0: the default)."""
         self._check(lib().pbf_set_wait_limit(self._h, int(reads)))
+
+    @property
+    def step_form(self) -> int:
+        """pbf_step_form: 0 a launch per phase, 1 to 4 the whole step in one launch."""
+        return lib().pbf_step_form(self._h)
 
     @property
     def stream(self) -> int:

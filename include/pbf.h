@@ -237,6 +237,9 @@ PBF_API pbf_status pbf_set_tuning(pbf_handle* h, const pbf_tuning* t);
 PBF_API pbf_status pbf_autotune(pbf_handle* h, double dt, int reps, pbf_tuning* out);
 
 PBF_API size_t pbf_size(const pbf_handle* h);
+/* The form of a step of this handle as its colliders are now: 0 a launch per phase, else one launch
+ * (1: one thread block cluster, 2 to 4: a cooperative grid). */
+PBF_API int pbf_step_form(const pbf_handle* h);
 PBF_API int pbf_num_scenes(const pbf_handle* h);
 
 /* Human-readable description of the last error on this handle (or of the
