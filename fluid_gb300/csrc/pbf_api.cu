@@ -286,6 +286,7 @@ pbf_status Handle::ensure_tape() {
 }
 
 pbf_status Handle::ensure_scratch(size_t bytes) {
+  close_surface();
   if (bytes <= scratch_bytes) return PBF_OK;
   if (scratch) cudaFree(scratch);
   scratch = nullptr;
@@ -340,6 +341,7 @@ pbf_status Handle::close_counts() {
 }
 
 pbf_status Handle::resort() {
+  close_surface();
   pbf_status st = usable();
   if (st == PBF_OK) st = close_counts();
   if (st == PBF_OK) st = cuda(launch_resort(b, dp, tune, cur, stream), "resort");
@@ -423,6 +425,7 @@ pbf_status Handle::enqueue_steps(float dt, int nsteps) {
   if (form == 0 && nsteps > 0) ok = close_counts();
   if (ok != PBF_OK) return ok;
   if (small_step_waits(form) && nsteps > 0) counts_open = true;
+  close_surface();
   const bool use_graph = (params.flags & PBF_FLAG_GRAPH) != 0;
   const bool keep_pred = b.pred != nullptr;
   const int it = params.iters;
@@ -706,6 +709,7 @@ pbf_status pbf_adjoint_step_device(pbf_handle* hh, double dt, const float* xyz, 
   st = h->join_from(static_cast<cudaStream_t>(stream));
   if (st == PBF_OK) st = h->close_counts();
   if (st != PBF_OK) return st;
+  h->close_surface();
   if (xyz) {
     st = h->cuda(pbf::launch_upload(h->b, h->cur, xyz, vel, nullptr, h->stream), "upload");
     if (st != PBF_OK) return st;
@@ -775,6 +779,7 @@ pbf_status pbf_set_state(pbf_handle* hh, const float* xyz, const float* vel) {
   pbf::DeviceGuard g(h->device);
   const size_t n = h->b.n;
   if (n == 0) return PBF_OK;
+  h->close_surface();
   pbf_status st = h->cuda(cudaMemcpyAsync(h->b.io, xyz, 3 * sizeof(float) * n, cudaMemcpyHostToDevice, h->stream),
                           "H2D");
   if (st == PBF_OK && vel)
@@ -791,6 +796,7 @@ pbf_status pbf_set_state_device(pbf_handle* hh, const float* xyz, const float* v
   Handle* h = reinterpret_cast<Handle*>(hh);
   if (!xyz && h->b.n) return h->fail(PBF_ERR_INVALID, "xyz is NULL");
   pbf::DeviceGuard g(h->device);
+  h->close_surface();
   pbf_status st = h->join_from(static_cast<cudaStream_t>(stream));
   if (st == PBF_OK)
     st = h->cuda(pbf::launch_upload(h->b, h->cur, xyz, vel, nullptr, h->stream), "upload");
@@ -1118,32 +1124,52 @@ pbf_status Handle::surface_emit(const SurfGrid& g, double isolevel, float* xyz, 
 
 }  // namespace pbf
 
-pbf_status pbf_surface(pbf_handle* hh, double isolevel, double step, const double* lo, const double* hi,
-                       float* xyz, float* nrm, size_t cap, size_t* count) {
+pbf_status pbf_surface_begin(pbf_handle* hh, double isolevel, double step, const double* lo, const double* hi,
+                             size_t* count) {
   if (!hh) return PBF_ERR_INVALID;
   Handle* h = reinterpret_cast<Handle*>(hh);
   if (!count) return h->fail(PBF_ERR_INVALID, "count is NULL");
-  if (cap && (!xyz || !nrm)) return h->fail(PBF_ERR_INVALID, "xyz / nrm is NULL");
   *count = 0;
   pbf::DeviceGuard dg(h->device);
-  pbf::SurfGrid g;
   uint32_t total = 0;
-  pbf_status st = h->surface_count(isolevel, step, lo, hi, &g, &total);
+  h->close_surface();
+  pbf_status st = h->surface_count(isolevel, step, lo, hi, &h->surf_grid, &total);
   if (st != PBF_OK) return st;
+  h->surf_open = true;
+  h->surf_iso = isolevel;
+  h->surf_total = total;
   *count = total;
-  const size_t m = std::min(static_cast<size_t>(total), cap);
+  return PBF_OK;
+}
+
+pbf_status pbf_surface_end(pbf_handle* hh, float* xyz, float* nrm, size_t cap) {
+  if (!hh) return PBF_ERR_INVALID;
+  Handle* h = reinterpret_cast<Handle*>(hh);
+  if (cap && (!xyz || !nrm)) return h->fail(PBF_ERR_INVALID, "xyz / nrm is NULL");
+  if (!h->surf_open) return h->fail(PBF_ERR_INVALID, "no surface begun, or the handle was used since");
+  pbf::DeviceGuard dg(h->device);
+  h->close_surface();
+  const size_t m = std::min(static_cast<size_t>(h->surf_total), cap);
   if (m == 0) return PBF_OK;
   if (m > (size_t(1) << 28)) return h->fail(PBF_ERR_INVALID, "surface too large: more than 2^28 triangles");
-  st = h->ensure_surface_out(sizeof(float) * 18 * m);
+  pbf_status st = h->ensure_surface_out(sizeof(float) * 18 * m);
   if (st != PBF_OK) return st;
   float* dev = h->surf_out;
-  st = h->surface_emit(g, isolevel, dev, dev + 9 * m, static_cast<uint32_t>(m));
+  st = h->surface_emit(h->surf_grid, h->surf_iso, dev, dev + 9 * m, static_cast<uint32_t>(m));
   if (st == PBF_OK)
     st = h->cuda(cudaMemcpyAsync(xyz, dev, sizeof(float) * 9 * m, cudaMemcpyDeviceToHost, h->stream), "D2H");
   if (st == PBF_OK)
     st = h->cuda(cudaMemcpyAsync(nrm, dev + 9 * m, sizeof(float) * 9 * m, cudaMemcpyDeviceToHost, h->stream), "D2H");
   if (st == PBF_OK) st = h->cuda(cudaStreamSynchronize(h->stream), "sync");
   return st;
+}
+
+pbf_status pbf_surface(pbf_handle* hh, double isolevel, double step, const double* lo, const double* hi,
+                       float* xyz, float* nrm, size_t cap, size_t* count) {
+  if (!hh) return PBF_ERR_INVALID;
+  if (cap && (!xyz || !nrm)) return reinterpret_cast<Handle*>(hh)->fail(PBF_ERR_INVALID, "xyz / nrm is NULL");
+  pbf_status st = pbf_surface_begin(hh, isolevel, step, lo, hi, count);
+  return st == PBF_OK ? pbf_surface_end(hh, xyz, nrm, cap) : st;
 }
 
 pbf_status pbf_estimate_density_at(pbf_handle* hh, size_t m, const float* pts, float* out) {
@@ -1315,6 +1341,7 @@ pbf_status pbf_restore(pbf_handle* hh) {
   Handle* h = reinterpret_cast<Handle*>(hh);
   if (!h->snap_valid) return h->fail(PBF_ERR_INVALID, "no snapshot taken");
   pbf::DeviceGuard g(h->device);
+  h->close_surface();
   const size_t m = h->b.n;
   pbf_status st =
       h->cuda(cudaMemcpyAsync(h->b.pos[h->cur], h->snap_pos, sizeof(float4) * m, cudaMemcpyDeviceToDevice, h->stream), "copy");

@@ -65,6 +65,12 @@ struct Handle {
   size_t surf_hash_bytes = 0;
   float* surf_out = nullptr;            // grow-only: the triangles of pbf_surface before their copy to the host
   size_t surf_out_bytes = 0;
+  // the surface that pbf_surface_begin counted and pbf_surface_end has not written: its grid and
+  // counts are in scratch, of the state as it is (close_surface: what changes either)
+  bool surf_open = false;
+  SurfGrid surf_grid{};
+  double surf_iso = 0;
+  uint32_t surf_total = 0;
   float4* mesh_dev = nullptr;           // collider triangles and their hierarchy (pbf_set_collider_mesh)
   float4* sph_dev = nullptr;            // collider spheres (pbf_set_collider_spheres)
   RenderState render;                   // path tracer (pbf_render_set_scene, pbf_render)
@@ -87,6 +93,7 @@ struct Handle {
   pbf_status enqueue_steps(float dt, int nsteps);
   pbf_status sync_and_check();
   pbf_status usable();        // PBF_ERR_TIMEOUT once a wait is known to have given up
+  void close_surface() { surf_open = false; }
   pbf_status close_counts();  // before a per-phase kernel counts into the cells
   pbf_status resort();        // the current state into cell order
   void drop_graphs();

@@ -133,6 +133,8 @@ def _declare(L):
         "pbf_density_noalloc": (st, [P, sz, P, P, P]),
         "pbf_adjoint_step_device": (st, [P, ctypes.c_double, P, P, P, P, P, P, P, P, P, P]),
         "pbf_surface": (st, [P, ctypes.c_double, ctypes.c_double, P, P, P, P, sz, P]),
+        "pbf_surface_begin": (st, [P, ctypes.c_double, ctypes.c_double, P, P, P]),
+        "pbf_surface_end": (st, [P, P, P, sz]),
         "pbf_mc_table": (None, [P, P, P]),
         "pbf_set_collider_mesh": (st, [P, sz, P]),
         "pbf_set_collider_spheres": (st, [P, sz, P]),
@@ -351,20 +353,11 @@ class Simulator:
         lo_a = None if lo is None else np.ascontiguousarray(lo, dtype=np.float64)
         hi_a = None if hi is None else np.ascontiguousarray(hi, dtype=np.float64)
         count = ctypes.c_size_t(0)
-        # One call when the triangles fit the room made for them (a surface grows with the square of
-        # the cubes across the particles' extent; pages that stay untouched cost nothing), else a
-        # second one with the room the first reported.
-        room = 4096 + int(48.0 * (0.5 * self.params.h / step) ** 2 * self.n ** (2.0 / 3.0)) if step > 0 else 4096
-        room = min(room, 1 << 26)
-        while True:
-            xyz = np.empty((room, 3, 3), dtype=np.float32)
-            nrm = np.empty((room, 3, 3), dtype=np.float32)
-            self._check(lib().pbf_surface(self._h, iso, step, _ptr(lo_a), _ptr(hi_a), _ptr(xyz), _ptr(nrm), room,
-                                          ctypes.byref(count)))
-            t = count.value
-            if t <= room:
-                return xyz[:t], nrm[:t]
-            room = t
+        self._check(lib().pbf_surface_begin(self._h, iso, step, _ptr(lo_a), _ptr(hi_a), ctypes.byref(count)))
+        xyz = np.empty((count.value, 3, 3), dtype=np.float32)
+        nrm = np.empty((count.value, 3, 3), dtype=np.float32)
+        self._check(lib().pbf_surface_end(self._h, _ptr(xyz), _ptr(nrm), count.value))
+        return xyz, nrm
 
     def set_render_scene(self, scene):
         """The scene the fluid is rendered in (a fluid_gb300.render.RenderScene)."""

@@ -289,6 +289,13 @@ PBF_API pbf_status pbf_adjoint_step_device(pbf_handle* h, double dt, const float
  */
 PBF_API pbf_status pbf_surface(pbf_handle* h, double isolevel, double step, const double* lo, const double* hi,
                                float* xyz, float* nrm, size_t cap, size_t* count);
+/* pbf_surface in two parts, for a caller that makes its room by the count: begin counts, end writes
+ * the first min(cap, total) triangles of the surface begun last (once; PBF_ERR_INVALID when the handle's
+ * state was stepped, set or queried in between). Each handle keeps device memory for its largest
+ * surface until it is destroyed: 72 bytes a triangle beside the grid's field and the normals' table. */
+PBF_API pbf_status pbf_surface_begin(pbf_handle* h, double isolevel, double step, const double* lo,
+                                     const double* hi, size_t* count);
+PBF_API pbf_status pbf_surface_end(pbf_handle* h, float* xyz, float* nrm, size_t cap);
 
 /*
  * pbf_set_collider_mesh -- triangles the particles collide with besides the box walls,
