@@ -87,3 +87,17 @@ def test_forms_of_handles():
                 assert sim.step_form == 0
                 sim.set_collider_spheres(None)
                 assert sim.step_form == form
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 33, 64, 65, 500, 700, 1024, 1025, 3000, 9727, 9729, 12000, 19455, 19457, 38911])
+def test_the_scenes_of_the_bit_comparison_take_the_whole_step_kernel(n):
+    import torch
+
+    from fluid_gb300 import pbf, scenes
+    from tests.test_gpu_small_step import _state
+
+    pos, vel, h = _state(n, seed=n)
+    fits = n <= 256 * torch.cuda.get_device_properties(0).multi_processor_count
+    with pbf.Simulator(pos, vel, scenes.physical_params(h, h / 2, max_neighbors=256)) as sim:
+        assert (sim.step_form > 0) == fits
