@@ -53,7 +53,7 @@ UNIT = "particle-updates/s"
 ALGO_BYTES = {"predict": 64 + 24, "sort": 104, "gather": 0, "lambda": 20, "deltap": 36,
               "xsph": 84, "vorticity": 64, "neighbors": 16, "scan": 0, "stats": 0}
 # DRAM bytes per particle per launch measured by ncu (dram__bytes_read.sum +
-# dram__bytes_write.sum) on the 1M colliding-blocks scene: profiles/colliding_blocks_1m_launch_list.md.
+# dram__bytes_write.sum) on the 1M colliding-blocks scene.
 PER_ITERATION = ("lambda", "deltap")  # phases launched once per Jacobi iteration
 NCU_TRAFFIC_PER_PARTICLE: dict[str, float] = {"deltap": 139.5, "lambda": 96.5, "neighbors": 56.2}
 

@@ -12,9 +12,10 @@ namespace pbf {
 // Programmatic dependent launch. Every kernel of the step's chains begins with chain_begin(): it
 // waits until the kernel before has finished and its writes are visible. All threads call it before
 // anything else, so a kernel is done only after the one before it. What it hides is the launch
-// itself: 33k particles with a mesh 258 -> 219 us a step, the adjoint of 262k 767 -> 711. A kernel
-// lets the next one's blocks in only when its own are done: let in earlier (launch_dependents at
-// the start of a kernel), they hold the places of blocks that could work (1M: 806 -> 1,236 us).
+// itself (us of calls enqueued back to back): a step of 33k particles with a mesh 258 -> 219, the
+// adjoint of 262k 767 -> 711. A kernel lets the next one's blocks in only when its own are done: let in
+// earlier (launch_dependents at the start of a kernel), they hold the places of blocks that could work
+// (1M: 806 -> 1,236 us).
 __device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Launches such a kernel behind the one before it in the stream.
 template <typename... Params, typename... Args>
@@ -64,13 +65,6 @@ __device__ __forceinline__ float square_rn(const float3 a) {
 // x* = fl(x + displacement), one rounding per component wherever it is formed.
 __device__ __forceinline__ float3 displaced(const float3 x, const float3 d) {
   return make_float3(__fadd_rn(x.x, d.x), __fadd_rn(x.y, d.y), __fadd_rn(x.z, d.z));
-}
-
-// Exactly rounded |a - b|^2 with no contraction: the neighbour predicate of
-// particles.cpp:260 evaluated in FP32 (a host check can repeat it bit for bit).
-__device__ __forceinline__ float dist2_rn(const float4& a, const float4& b) {
-  const float dx = __fsub_rn(a.x, b.x), dy = __fsub_rn(a.y, b.y), dz = __fsub_rn(a.z, b.z);
-  return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
 }
 
 // Cell of x* within its scene's grid: floor((x - origin) * inv_cell), clamped.
@@ -564,8 +558,8 @@ __device__ __forceinline__ void collide_reverse(uint32_t code, const float3 p, c
 // they lie in the rows dy = -1..1 of cells cx-1..cx+1, all within 2*nx+3 cells after the
 // slab's first candidate cell, i.e. a short slot range of the cell-sorted arrays. A
 // neighbour is stored as a u16 entry (slab << 14 | slot offset from the slab's first
-// candidate slot), two entries per u32 word, word-major ([word][N]) so a warp's loads of
-// one word index coalesce. hdr = {slab base -1, slab base 0, slab base +1, count}.
+// candidate slot), two entries per u32 word, the words in groups of four (list_word); the
+// header is nbr_decode's.
 constexpr int kOffsetBits = 14;
 constexpr uint32_t kOffsetMask = (1u << kOffsetBits) - 1u;
 
@@ -575,22 +569,13 @@ __device__ __forceinline__ int nbr_total(const uint4& h) { return static_cast<in
 // header holds slab 0's first slot in x and, in y and z, slab 1's and slab 2's first slots
 // less slab 0's and less the tag bits (g << 14), all modulo 2^32, so the slot is
 // x + entry + (0, y or z by tag): the entry needs no masking.
-// Two forms of the same decode (slab tags are 0, 1 and 2, so both give the same slot).
-// The compiler schedules a pass's gathers differently around them; every pass measured
-// fastest with kBits on the 1M colliding blocks (ms per step, kBits / kCompare): lambda
-// 0.238 / 0.256 and delta-p 0.282 / 0.315 with word-major lists, XSPH 0.084 / 0.100 with
-// the grouped list words.
-enum class Decode { kBits, kCompare };
-
-template <Decode DC = Decode::kBits>
+// The tag is taken by bit tests, and the header's part is a value of its own: the compiler schedules a
+// pass's gathers around the decode. By comparing the tag, ms per step on the 1M colliding blocks: lambda
+// 0.256 against 0.238 and delta-p 0.315 against 0.282 with word-major lists, XSPH 0.100 against 0.084
+// with the grouped list words; the same bit tests inside the sum: 33k particles on a mesh 222.6 against
+// 219.5 us a step.
 __device__ __forceinline__ uint32_t nbr_decode(const uint4& h, uint32_t e) {
-  uint32_t adj;
-  if (DC == Decode::kBits) {
-    adj = (e & (2u << kOffsetBits)) ? h.z : ((e & (1u << kOffsetBits)) ? h.y : 0u);
-  } else {
-    const uint32_t g = e >> kOffsetBits;
-    adj = g == 0u ? 0u : (g == 1u ? h.y : h.z);
-  }
+  const uint32_t adj = (e & (2u << kOffsetBits)) ? h.z : ((e & (1u << kOffsetBits)) ? h.y : 0u);
   return h.x + e + adj;
 }
 
@@ -621,7 +606,7 @@ __device__ __forceinline__ void for_each_neighbor(int i, int n, const uint4 h,
 // gathers in flight. A round of 8 entries is one 16-byte group of list words; with D = 8
 // the next group is loaded before this round's computation, so its latency overlaps it.
 // The last group, with fewer than 8 entries left, is taken from the same registers. Calls
-// f(j, load(j)) in the same (ascending) order. D = 4 or 8; DC picks the decode form.
+// f(j, load(j)) in the same (ascending) order. D = 4 or 8.
 // List words are read once per pass: ST = true loads them with the streaming policy
 // (ld.global.cs, evict-first in L1 and L2), so they displace less of the neighbours' x*
 // that the pass gathers repeatedly.
@@ -634,7 +619,7 @@ __device__ __forceinline__ uint4 ld_hdr(const uint4* p) {
   return ST ? __ldcs(p) : __ldg(p);
 }
 
-template <int D, Decode DC = Decode::kBits, bool ST = false, typename L, typename F>
+template <int D, bool ST = false, typename L, typename F>
 __device__ __forceinline__ void for_each_neighbor_pf(int i, int n, const uint4 h,
                                                      const uint32_t* __restrict__ words, L&& load, F&& f) {
   static_assert(D == 4 || D == 8, "gather depth 4 or 8");
@@ -648,11 +633,11 @@ __device__ __forceinline__ void for_each_neighbor_pf(int i, int n, const uint4 h
     qp += sn;
     uint4 nq = make_uint4(0u, 0u, 0u, 0u);
     if (D == 8 && k + 8 < total) nq = ld_quad<ST>(qp);
-    const uint32_t j0 = nbr_decode<DC>(h, q.x & 0xffffu), j1 = nbr_decode<DC>(h, q.x >> 16);
-    const uint32_t j2 = nbr_decode<DC>(h, q.y & 0xffffu), j3 = nbr_decode<DC>(h, q.y >> 16);
+    const uint32_t j0 = nbr_decode(h, q.x & 0xffffu), j1 = nbr_decode(h, q.x >> 16);
+    const uint32_t j2 = nbr_decode(h, q.y & 0xffffu), j3 = nbr_decode(h, q.y >> 16);
     if (D == 8) {
-      const uint32_t j4 = nbr_decode<DC>(h, q.z & 0xffffu), j5 = nbr_decode<DC>(h, q.z >> 16);
-      const uint32_t j6 = nbr_decode<DC>(h, q.w & 0xffffu), j7 = nbr_decode<DC>(h, q.w >> 16);
+      const uint32_t j4 = nbr_decode(h, q.z & 0xffffu), j5 = nbr_decode(h, q.z >> 16);
+      const uint32_t j6 = nbr_decode(h, q.w & 0xffffu), j7 = nbr_decode(h, q.w >> 16);
       const auto a0 = load(j0);
       const auto a1 = load(j1);
       const auto a2 = load(j2);
@@ -679,8 +664,8 @@ __device__ __forceinline__ void for_each_neighbor_pf(int i, int n, const uint4 h
       f(j1, a1);
       f(j2, a2);
       f(j3, a3);
-      const uint32_t j4 = nbr_decode<DC>(h, q.z & 0xffffu), j5 = nbr_decode<DC>(h, q.z >> 16);
-      const uint32_t j6 = nbr_decode<DC>(h, q.w & 0xffffu), j7 = nbr_decode<DC>(h, q.w >> 16);
+      const uint32_t j4 = nbr_decode(h, q.z & 0xffffu), j5 = nbr_decode(h, q.z >> 16);
+      const uint32_t j6 = nbr_decode(h, q.w & 0xffffu), j7 = nbr_decode(h, q.w >> 16);
       const auto a4 = load(j4);
       const auto a5 = load(j5);
       const auto a6 = load(j6);
@@ -694,8 +679,8 @@ __device__ __forceinline__ void for_each_neighbor_pf(int i, int n, const uint4 h
   }
   // fewer than 8 entries left, all in q
   if (k + 3 < total) {
-    const uint32_t j0 = nbr_decode<DC>(h, q.x & 0xffffu), j1 = nbr_decode<DC>(h, q.x >> 16);
-    const uint32_t j2 = nbr_decode<DC>(h, q.y & 0xffffu), j3 = nbr_decode<DC>(h, q.y >> 16);
+    const uint32_t j0 = nbr_decode(h, q.x & 0xffffu), j1 = nbr_decode(h, q.x >> 16);
+    const uint32_t j2 = nbr_decode(h, q.y & 0xffffu), j3 = nbr_decode(h, q.y >> 16);
     const auto a0 = load(j0);
     const auto a1 = load(j1);
     const auto a2 = load(j2);
@@ -709,7 +694,7 @@ __device__ __forceinline__ void for_each_neighbor_pf(int i, int n, const uint4 h
     q.y = q.w;
   }
   if (k + 1 < total) {
-    const uint32_t j0 = nbr_decode<DC>(h, q.x & 0xffffu), j1 = nbr_decode<DC>(h, q.x >> 16);
+    const uint32_t j0 = nbr_decode(h, q.x & 0xffffu), j1 = nbr_decode(h, q.x >> 16);
     const auto a0 = load(j0);
     const auto a1 = load(j1);
     f(j0, a0);
@@ -718,18 +703,9 @@ __device__ __forceinline__ void for_each_neighbor_pf(int i, int n, const uint4 h
     q.x = q.y;
   }
   if (k < total) {
-    const uint32_t j0 = nbr_decode<DC>(h, q.x & 0xffffu);
+    const uint32_t j0 = nbr_decode(h, q.x & 0xffffu);
     f(j0, load(j0));
   }
-}
-
-// The common case: the neighbours' x* (NC: through the read-only path, for buffers no
-// thread writes during the kernel), four in flight; calls f(j, x_j).
-template <bool NC, typename F>
-__device__ __forceinline__ void for_each_neighbor_x(int i, int n, const uint4 h,
-                                                    const uint32_t* __restrict__ words,
-                                                    const float4* xs, F&& f) {
-  for_each_neighbor_pf<4>(i, n, h, words, [&](uint32_t j) -> float4 { return NC ? __ldg(&xs[j]) : xs[j]; }, f);
 }
 
 // Pair geometry shared by every neighbour pass, branch-free:
@@ -740,40 +716,24 @@ struct Pair {
   float3 r;
   float r2, q, s;
 };
-// FTZ selects the flush-to-zero form of the approximate reciprocal square root, which
-// needs no rescaling of subnormal inputs. The two forms differ only for a subnormal r2,
-// far below EPS_D^2, where s is 0 either way (and both give +inf at r2 = 0, where hr is 0),
-// so the pair values are the same. Every pass uses it: measured with the current kernels on
-// the 1M colliding blocks, lambda 0.222 against 0.235 ms a step, delta-p 0.274 against
-// 0.279, XSPH 0.090 against 0.093 (the vorticity pass already used it).
+// The approximate reciprocal square root is the flush-to-zero form, which needs no rescaling of
+// subnormal inputs. The other form differs only for a subnormal r2, far below EPS_D^2, where s is 0
+// either way (and both give +inf at r2 = 0, where hr is 0), so the pair values are the same: on the 1M
+// colliding blocks lambda 0.222 against 0.235 ms a step, delta-p 0.274 against 0.279, XSPH 0.090
+// against 0.093.
 // Every rounding is explicit (_rn intrinsics, fused where written as an fma), so the
 // compiler cannot contract differently in differently unrolled loops: every form of a
 // neighbour pass gives the same bits.
-template <bool FTZ = true>
 __device__ __forceinline__ Pair pair_of(const float4& xi, const float4& xj, float h, float h2) {
   Pair p;
   p.r = make_float3(__fsub_rn(xi.x, xj.x), __fsub_rn(xi.y, xj.y), __fsub_rn(xi.z, xj.z));
   p.r2 = __fmaf_rn(p.r.z, p.r.z, __fmaf_rn(p.r.y, p.r.y, __fmul_rn(p.r.x, p.r.x)));
   p.q = fmaxf(__fsub_rn(h2, p.r2), 0.0f);
   float rinv;
-  if (FTZ)
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rinv) : "f"(p.r2));
-  else
-    rinv = rsqrtf(p.r2);
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rinv) : "f"(p.r2));
   const float hr = fmaxf(__fmaf_rn(-p.r2, rinv, h), 0.0f);
   p.s = p.r2 >= kEps * kEps ? __fmul_rn(__fmul_rn(hr, hr), rinv) : 0.0f;
   return p;
-}
-
-// Spiky gradient factor s with grad W(r) = spiky_c * s * r (particles.cpp:143-149);
-// returns false outside [EPS_D, h).
-__device__ __forceinline__ bool spiky_s(float r2, float h, float* s) {
-  const float rinv = rsqrtf(r2);
-  const float rl = r2 * rinv;
-  if (!(rl < h && rl >= kEps)) return false;
-  const float hr = h - rl;
-  *s = hr * hr * rinv;
-  return true;
 }
 
 // Particles::estimateDensityAt (particles.cpp:446-453): sum of poly6 over all particles

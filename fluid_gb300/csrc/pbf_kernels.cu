@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(BLOCK) k_lambda(float4* xs, const uint4* __res
   const float4 xi = xs[i];
   LambdaSum sum;
   // D gathers in flight
-  for_each_neighbor_pf<D, Decode::kBits, ST>(i, n, ld_hdr<ST>(&hdr[i]), words,
+  for_each_neighbor_pf<D, ST>(i, n, ld_hdr<ST>(&hdr[i]), words,
                                               [&](uint32_t j) -> float4 { return xs[j]; },
                                               [&](uint32_t, const float4& xj) { sum.add(xi, xj, P); });
   float rho;
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(BLOCK) k_deltap(const float4* __restrict__ xs,
   const float4 xi = xs[i];
   const float wt = P.poly6_c * P.tis;
   DeltaSum<N4> sum;  // lambda_i is x*_i.w
-  for_each_neighbor_pf<D, Decode::kBits, ST>(i, n, ld_hdr<ST>(&hdr[i]), words,
+  for_each_neighbor_pf<D, ST>(i, n, ld_hdr<ST>(&hdr[i]), words,
                                               [&](uint32_t j) -> float4 { return __ldg(&xs[j]); },
                                               [&](uint32_t, const float4& xj) { sum.add(xi, xj, wt, P); });
   const float3 dp = sum.delta(P);
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(BLOCK) k_xsph(float4* xs, const float4* __rest
   const float4 xi = xs[i];
   const float3 vi = f3(disp[i]) * inv_dt;  // updateVelocity, particles.cpp:215-217
   XsphSum sum;
-  for_each_neighbor_pf<D, Decode::kBits, ST>(
+  for_each_neighbor_pf<D, ST>(
       i, n, ld_hdr<ST>(&hdr[i]), words, [&](uint32_t j) { return XD{xs[j], __ldg(&disp[j])}; },
       [&](uint32_t, const XD& a) { sum.add(xi, vi, a, inv_dt, P); });
   const float3 v = sum.velocity(vi, P);
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(BLOCK) k_vort(const float4* __restrict__ xs,
   if (i >= n) return;
   const float4 xi = xs[i];
   VortSum sum;  // |omega_j| is x*_j.w
-  for_each_neighbor_pf<D, Decode::kBits, ST>(i, n, ld_hdr<ST>(&hdr[i]), words,
+  for_each_neighbor_pf<D, ST>(i, n, ld_hdr<ST>(&hdr[i]), words,
                                               [&](uint32_t j) -> float4 { return __ldg(&xs[j]); },
                                               [&](uint32_t, const float4& xj) { sum.add(xi, xj, P); });
   const float3 eta = sum.location(P);

@@ -87,7 +87,8 @@ __device__ __noinline__ void nbr_scan_thread(int i, const float4* xs, const floa
       // one reaching below x - W) finds the first candidate at or above x - W, and the
       // first one above x + W ends the row (W = w cells, margin included; with NaN
       // coordinates in the cell the search may start early, never late). The predicate
-      // reuses the x difference: the same roundings as dist2_rn. The own slot is a hit at
+      // reuses the x difference. Every difference and square is rounded, |x*_i - x*_j|^2 <= H2
+      // of particles.cpp:260 as a host check repeats it. The own slot is a hit at
       // distance 0 and is dropped there, which keeps one loop per row (two half-row loops
       // around it: 0.209 against 0.206 ms; one loop over a slab's three rows, lanes moving
       // on to the next row when theirs ends: 0.243 against 0.234 ms, 48 registers).
@@ -131,8 +132,8 @@ __device__ __noinline__ void nbr_scan_thread(int i, const float4* xs, const floa
 // the candidates of all of them are, in each of the 9 rows around theirs, one slot range (cells
 // one before the first to one after the last, trimmed by binary search to the x reach). The
 // ranges are read as one flat list, 32 candidates a turn, one per lane; a turn tests its 32
-// candidates against the group's slots, two slots at a time in packed FP32x2 (the roundings of
-// dist2_rn), and each slot's 32 results are one ballot word in shared memory. Then each lane
+// candidates against the group's slots, two slots at a time in packed FP32x2 (the thread
+// scan's roundings), and each slot's 32 results are one ballot word in shared memory. Then each lane
 // turns the words of its own slot into list entries, in ascending slot order as the thread scan
 // appends them, all lanes at the same entry index: 8 entries make one 16-byte store, and a warp's
 // stores are contiguous. The lists (neighbours and their order) are the thread scan's.

@@ -233,6 +233,8 @@ PBF_API pbf_status pbf_set_tuning(pbf_handle* h, const pbf_tuning* t);
  * CUDA events over `reps` steps of dt from the current state (checkpointed
  * and restored around every trial, so the state is unchanged on return),
  * keeps the fastest candidate per dimension and reports the result in *out (may be NULL).
+ * On a small scene it times the launches per phase, which its recorded (adjoint) and profiled
+ * steps take, not the one launch of its other steps.
  */
 PBF_API pbf_status pbf_autotune(pbf_handle* h, double dt, int reps, pbf_tuning* out);
 
